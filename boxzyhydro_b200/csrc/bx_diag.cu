@@ -55,21 +55,62 @@ __global__ void k_divcheck(unsigned long long n, unsigned long long seed, int er
     const bool ok1 = __double_as_longlong(q) == __double_as_longlong(ref) || (q == 0.0 && ref == 0.0);
     // cdiv serves grid constants, which bx_create keeps inside [2^-450, 2^450]
     const bool in_window = d >= 0x1p-450 && d <= 0x1p+450;
+    bool ok4 = true;
+    if (bx::den_fast_ok(d))
+      ok4 = __double_as_longlong(bx::rcp_fast(d)) == __double_as_longlong(1.0 / d);
     const bool ok2 = !in_window || __double_as_longlong(q2) == __double_as_longlong(ref) ||
                      (q2 == 0.0 && ref == 0.0);
     // the HLL form: every bit of the IEEE quotient, the sign of a zero included,
     // wherever quot_fast_ok admits the numerator and d lies in the window
     bool ok3 = true;
-    if (in_window && bx::quot_fast_ok(a)) {
-      const double q3 = bx::quot_fast(a, d, __drcp_rn(d));
+    if (bx::den_fast_ok(d) && bx::quot_fast_ok(a)) {
+      const double q3 = bx::quot_fast(a, d, bx::rcp_fast(d));
       ok3 = __double_as_longlong(q3) == __double_as_longlong(ref);
     }
-    if (!(ok1 && ok2 && ok3)) {
+    if (!(ok1 && ok2 && ok3 && ok4)) {
       if (atomicAdd(bad, 1ull) == 0) { example[0] = a; example[1] = d; }
     }
   }
 }
+
+// sqrt_fast against the IEEE square root: the n given arguments, then `nrandom`
+// random ones with exponents in [-e, e]
+__global__ void k_rootcheck(const double* q, unsigned long long n, unsigned long long nrandom,
+                            unsigned long long seed, int erange, unsigned long long* bad,
+                            double* example) {
+  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
+  for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+       i < n + nrandom; i += stride) {
+    const double x = i < n ? q[i] : rnd(mix(seed ^ i), erange, false);
+    if (__double_as_longlong(bx::sqrt_fast(x)) != __double_as_longlong(sqrt(x)))
+      if (atomicAdd(bad, 1ull) == 0) example[0] = x;
+  }
+}
 }  // namespace
+
+extern "C" int bx_check_root(const double* q, unsigned long long n, unsigned long long nrandom,
+                             unsigned long long seed, int exp_range,
+                             unsigned long long* mismatches, double* example) {
+  if ((n && !q) || exp_range < 0 || exp_range > 900) return 1;
+  double* d = nullptr;
+  unsigned long long* bad = nullptr;
+  const size_t bytes = n * sizeof(double);
+  if (cudaMalloc(&d, bytes + sizeof(double)) != cudaSuccess) return 5;
+  if (cudaMalloc(&bad, sizeof(*bad)) != cudaSuccess) { cudaFree(d); return 5; }
+  cudaMemset(bad, 0, sizeof(*bad));
+  cudaMemset(d + n, 0, sizeof(double));
+  if (n) cudaMemcpy(d, q, bytes, cudaMemcpyHostToDevice);
+  k_rootcheck<<<1184, 256>>>(d, n, nrandom, seed, exp_range, bad, d + n);
+  unsigned long long h = 0;
+  double hx = 0.0;
+  cudaMemcpy(&h, bad, sizeof(h), cudaMemcpyDeviceToHost);
+  cudaMemcpy(&hx, d + n, sizeof(hx), cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  cudaFree(bad);
+  if (mismatches) *mismatches = h;
+  if (example) *example = hx;
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
 
 extern "C" int bx_check_shared_division(unsigned long long n, unsigned long long seed,
                                          int exp_range, unsigned long long* mismatches,

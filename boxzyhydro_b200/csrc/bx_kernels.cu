@@ -229,13 +229,15 @@ __device__ __forceinline__ Raw load_raw(const StageArgs& a, const Geom& g, int x
 // residual correction (exact).  The corrections are valid while the numerators'
 // exponents lie in their window; one check of all of them at the end, rather
 // than a branch per division, and false sends the caller to prim_ieee.
-template <int STAGE>
+// LIB: with the library's reciprocal and root (the flux_ang instances, which
+// spill; the short forms' chains side by side would add to it).
+template <int STAGE, bool LIB = false>
 __device__ __forceinline__ bool prim_fast(const Geom& g, const Cons& c, double v1, double v2,
                                           double v3, int nsrc, bool need_c, Prim& q, int rs = 0) {
   const bool is0 = stage_is0<STAGE>(rs);
   const double d = c.d;
-  bool ok = d >= 0x1p-450 && d <= 0x1p+450;
-  const double r = ok ? __drcp_rn(d) : 1.0;
+  bool ok = den_fast_ok(d);
+  const double r = LIB ? (ok ? __drcp_rn(d) : 1.0) : rcp_fast(d);
   double E = c.E;
   if (is0) {
     // source(): E = max(E - K, eps) + K with K = half*|m|^2/rho, the same K each time
@@ -254,8 +256,9 @@ __device__ __forceinline__ bool prim_fast(const Geom& g, const Cons& c, double v
   q.c = 0.0;
   if (need_c) {
     const double pn = q.p * g.gam;
-    ok = ok && quot_fast_ok(pn);
-    q.c = sqrt(quot_fast(pn, d, r));
+    ok = ok && rad_fast_ok(pn);
+    const double qc = quot_fast(pn, d, r);
+    q.c = LIB ? sqrt(qc) : sqrt_fast(qc);
   }
   return ok;
 }
@@ -278,7 +281,7 @@ __device__ __forceinline__ Prim prim_ieee(double small_eps, double gm1, double g
   return q;
 }
 
-template <int STAGE, bool GRAV = false, bool TAB = false>
+template <int STAGE, bool GRAV = false, bool TAB = false, bool ANG = false>
 __device__ __forceinline__ Prim prim_of(const Geom& g, Raw r, unsigned& flags, int nsrc,
                                         double dth, bool need_c = true, int rs = 0,
                                         const EosDev* eos = nullptr) {
@@ -298,7 +301,7 @@ __device__ __forceinline__ Prim prim_of(const Geom& g, Raw r, unsigned& flags, i
     q.p = eos_pressure(q.d, c.E, v1, v2, v3, g.gm1, g.small_eps);
     // the sound speed enters only the lambdas of cells whose face states are built
     q.c = need_c ? sqrt(qd(q.p * g.gam)) : 0.0;
-  } else if (!prim_fast<STAGE>(g, r.c, r.v1, r.v2, r.v3, nsrc, need_c && !TAB, q, rs)) {
+  } else if (!prim_fast<STAGE, ANG>(g, r.c, r.v1, r.v2, r.v3, nsrc, need_c && !TAB, q, rs)) {
     q = prim_ieee<STAGE>(g.small_eps, g.gm1, g.gam, r.c, r.v1, r.v2, r.v3, nsrc,
                          need_c && !TAB, rs);
   }
@@ -358,7 +361,7 @@ __device__ __forceinline__ Prim load_prim(const StageArgs& a, const Geom& g, int
                                           unsigned& flags, int nsrc, double dth,
                                           bool need_c = true, int rs = 0) {
   const Raw r = load_raw<STAGE, GRAV, CG>(a, g, x, y, z, rs);
-  Prim q = prim_of<STAGE, GRAV, TAB>(g, r, flags, nsrc, dth, need_c, rs, &a.eos);
+  Prim q = prim_of<STAGE, GRAV, TAB, ANG>(g, r, flags, nsrc, dth, need_c, rs, &a.eos);
   // with flux_ang the momenta reconstructed are the transformed ones (the
   // sources leave the momenta alone)
   if (ANG) ang_to(g, x, y, r.c.m1, r.c.m2, q.rm, q.am);
@@ -465,9 +468,9 @@ __device__ __forceinline__ bool epi_fast(const Geom& g, const double n[5], doubl
                                          double& u3, double& r0) {
   const double d = n[0];
   const double kn = kHalf * (n[1] * n[1] + n[2] * n[2] + n[3] * n[3]);
-  bool ok = d >= 0x1p-450 && d <= 0x1p+450 && quot_fast_ok(n[1]) && quot_fast_ok(n[2]) &&
+  bool ok = den_fast_ok(d) && quot_fast_ok(n[1]) && quot_fast_ok(n[2]) &&
             quot_fast_ok(n[3]) && quot_fast_ok(kn);
-  const double r = ok ? __drcp_rn(d) : 1.0;
+  const double r = rcp_fast(d);
   u1 = quot_fast(n[1], d, r);
   u2 = quot_fast(n[2], d, r);
   u3 = quot_fast(n[3], d, r);
@@ -475,8 +478,8 @@ __device__ __forceinline__ bool epi_fast(const Geom& g, const double n[5], doubl
   const double E3 = fmax(n[4] - ek, g.small_eps) + ek;
   const double pA = eos_pressure(d, E3, u1, u2, u3, g.gm1, g.small_eps);
   const double pn = g.gam * pA;
-  ok = ok && quot_fast_ok(pn);
-  const double sound = sqrt(quot_fast(pn, d, r));
+  ok = ok && rad_fast_ok(pn);
+  const double sound = sqrt_fast(quot_fast(pn, d, r));
   if (POW2)
     r0 = (sound + fabs(u1)) * g.idx + (sound + fabs(u2)) * g.idy + (sound + fabs(u3)) * g.idz;
   else

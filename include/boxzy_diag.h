@@ -27,6 +27,14 @@ int bx_check_shared_division(unsigned long long n, unsigned long long seed, int 
                              unsigned long long *mismatches, double *example_a,
                              double *example_d);
 
+/* Self-check of the branch-free square root of the stage kernels: the n given
+ * arguments (host array, values in [2^-900, 2^900]) and nrandom random ones with
+ * exponents in [-exp_range, exp_range] (exp_range <= 900) against the IEEE square
+ * root; returns the number that differ in any bit and one example. */
+int bx_check_root(const double *q, unsigned long long n, unsigned long long nrandom,
+                  unsigned long long seed, int exp_range, unsigned long long *mismatches,
+                  double *example);
+
 #ifdef __cplusplus
 }
 #endif
