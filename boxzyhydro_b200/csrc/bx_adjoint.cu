@@ -388,7 +388,7 @@ k_rdir(Geom g, const double* P, const double* lamL, double lscale, double dt, do
       }
       const double ud = DIR == 0 ? qc.u1 : DIR == 1 ? qc.u2 : qc.u3;
       muscl_states<POW2>(qc, ud, sl[0], sl[1], sl[2], sl[3], sl[4], sl[5], dt, ds, ids, mi, pl);
-      double lp = fmax(ud + qc.c, 0.0) * dt, lm = fmin(ud - qc.c, 0.0) * dt;
+      double lp = at_least(ud + qc.c, 0.0) * dt, lm = at_most(ud - qc.c, 0.0) * dt;
       if (POW2) { lp *= ids; lm *= ids; }
       else { lp = cdiv(lp, ds, ids); lm = cdiv(lm, ds, ids); }
       hm = kHalf * (-1.0 - lm);

@@ -51,11 +51,11 @@ __device__ __forceinline__ void hll_vjp(const FaceState& L, const FaceState& R, 
   // ap = max(0, vr+cr, vl+cl), am = max(0, -(vr-cr), -(vl-cl)), evaluated as the forward
   const double a1 = vr + cr, a2 = vl + cl;
   const double b1 = -(vr - cr), b2 = -(vl - cl);
-  const double t1 = fmax(0.0, a1);
-  const double ap = fmax(t1, a2);
+  const double t1 = at_least(a1, 0.0);
+  const double ap = at_least(a2, t1);
   const int sap = (a2 > t1) ? 2 : (a1 > 0.0 ? 1 : 0);
-  const double t2 = fmax(0.0, b1);
-  const double am = fmax(t2, b2);
+  const double t2 = at_least(b1, 0.0);
+  const double am = at_least(b2, t2);
   const int sam = (b2 > t2) ? 2 : (b1 > 0.0 ? 1 : 0);
   const double iD = rcp_deriv(ap + am);
   const double apm = ap * am;

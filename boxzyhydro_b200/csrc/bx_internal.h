@@ -74,36 +74,19 @@ struct Tile {
   int z0, z1;     // interior-relative z range [z0,z1) (for nz<6: plane range)
 };
 
-// Stage-kernel tile: TX x TY interior columns per block of NT threads (NT may
-// exceed the tile: the threads without a column of their own take halo work).
-// 32x8 in 256 threads measured 5 % faster on B200 than 16x14 in 256 threads
-// (although the latter fits the x/y face-state and face-flux phases into two
-// passes of the block instead of three: the wider rows load whole 256-byte
-// segments and need fewer halo columns) and 2 % faster than 32x16 in 512
-// threads (one block per SM: its barriers have no second block to hide them).
-#ifndef BX_TX
-#define BX_TX 32
-#endif
-#ifndef BX_TY
-#define BX_TY 8
-#endif
-#ifndef BX_NT
-#define BX_NT 256
-#endif
-constexpr int TX = BX_TX;
-constexpr int TY = BX_TY;
-constexpr int NT = BX_NT;
-static_assert(TX * TY <= NT && NT % 32 == 0, "tile larger than the block");
-
 // The stage kernels' tile shapes: TX_ x TY_ interior columns in a block of NT
-// threads, and the shared-memory layout that follows from them (per z plane:
-// primitives of the tile plus a two-cell halo, aliased with the x/y face
-// fluxes; x and y face states; per-thread z-pipeline slots).  Shape 0 is the
-// single-grid path's (TX x TY); the batched path's autotuner may pick shape 1.
+// threads (NT may exceed the tile: the threads without a column of their own take
+// halo cells), and the shared-memory layout that follows (per z plane: primitives
+// of the tile plus a two-cell halo; x and y face states, whose plus half the face
+// fluxes then take; per-thread z-pipeline slots).  Shape 0 is the single-grid
+// path's; the batched path's autotuner may pick shape 1.  32 x 8 columns in 256
+// threads, two blocks per SM: 16 x 14 in 256 measured 5 % slower, 32 x 16 in 512
+// (one block per SM, its barriers without a second block to hide them) 2 %.
+constexpr int kStageThreads = 256;
 template <int TX_, int TY_, int MODE_ = 0>
 struct TileShape {
   static constexpr int TX = TX_, TY = TY_;
-  static constexpr int NT = BX_NT;
+  static constexpr int NT = kStageThreads;
   // MODE 1 (TAB): the tabulated EOS, whose gamma is a reconstructed primitive;
   // MODE 2 (ANG): angular-momentum fluxing, whose radial and angular momenta
   // are reconstructed primitives and whose x/y face fluxes of the two momentum
@@ -123,13 +106,13 @@ struct TileShape {
   // (5 + 5) and the plus z-state carried to the next plane (NSF), kept in
   // shared memory so the x/y phases have the registers
   static constexpr int NZS = 10 + NSF;
-  // the face fluxes of the face and update phases alias the primitives
-  static constexpr int NR0 = (NPF * NP > NFQ * (NFX + NFY)) ? NPF * NP : NFQ * (NFX + NFY);
-  static constexpr int SMEM_DOUBLES = NR0 + 2 * NSF * NSX + 2 * NSF * NSY + NZS * NOWN;
+  // one 16-bit table entry per state item (stage_tile)
+  static constexpr int SMEM_DOUBLES = NPF * NP + 2 * NSF * (NSX + NSY) + NZS * NOWN +
+                                      (NSX + NSY + 3) / 4;
   static_assert(TX * TY <= NT && NT % 32 == 0, "tile larger than the block");
   static_assert(4 * (TX + TY) <= NT, "one halo cell per thread and plane at most");
 };
-using Shape0 = TileShape<TX, TY>;
+using Shape0 = TileShape<32, 8>;
 using Shape1 = TileShape<16, 16>;
 // the tabulated EOS and angular-momentum fluxing (single grids only): 32 x 6
 // columns, so the larger primitive and face-state sets still fit two blocks

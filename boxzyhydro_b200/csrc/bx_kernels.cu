@@ -120,50 +120,50 @@ struct Cons {
   double d, m1, m2, m3, E;
 };
 
+// where a cell's values are read (its own place, or its donor's for a face
+// ghost: the offset within a plane) and which momenta are reflected
+struct Place {
+  long long c;
+  bool fx, fy, fz;
+};
+__device__ __forceinline__ Place place_of(const Geom& g, int x, int y, int z) {
+  Place p{0, false, false, false};
+  const int xx = remap_axis(x, g.ax0, g.ax1, g.wall[0], g.wall[1], p.fx);
+  const int yy = remap_axis(y, g.ay0, g.ay1, g.wall[2], g.wall[3], p.fy);
+  const int zz = g.threed ? remap_axis(z, g.az0, g.az1, g.wall[4], g.wall[5], p.fz) : z;
+  p.c = g.base + xx + (long long)yy * g.sy + (long long)zz * g.sz;
+  return p;
+}
+
 template <bool CG = false>
-__device__ __forceinline__ Cons load_cons(const double* B, long long PS, const Geom& g, int x,
-                                          int y, int z) {
-  bool fx = false, fy = false, fz = false;
-  const int xx = remap_axis(x, g.ax0, g.ax1, g.wall[0], g.wall[1], fx);
-  const int yy = remap_axis(y, g.ay0, g.ay1, g.wall[2], g.wall[3], fy);
-  const int zz = g.threed ? remap_axis(z, g.az0, g.az1, g.wall[4], g.wall[5], fz) : z;
-  const long long c = g.base + xx + (long long)yy * g.sy + (long long)zz * g.sz;
+__device__ __forceinline__ Cons load_cons(const double* B, long long PS, const Place& p) {
+  const double* b = B + p.c;
   Cons r;
-  r.d = ldg<CG>(B + c);
-  r.m1 = ldg<CG>(B + PS + c);
-  r.m2 = ldg<CG>(B + 2 * PS + c);
-  r.m3 = ldg<CG>(B + 3 * PS + c);
-  r.E = ldg<CG>(B + 4 * PS + c);
-  if (fx) r.m1 = -r.m1;
-  if (fy) r.m2 = -r.m2;
-  if (fz) r.m3 = -r.m3;
+  r.d = ldg<CG>(b);
+  r.m1 = ldg<CG>(b + PS);
+  r.m2 = ldg<CG>(b + 2 * PS);
+  r.m3 = ldg<CG>(b + 3 * PS);
+  r.E = ldg<CG>(b + 4 * PS);
+  if (p.fx) r.m1 = -r.m1;
+  if (p.fy) r.m2 = -r.m2;
+  if (p.fz) r.m3 = -r.m3;
   return r;
 }
 
 // the step input's velocity m/rho at a cell, as stage 0 stored it for the
-// interior cells (ghost cells read their source cell, reflected components negated)
-template <bool CG = false>
-__device__ __forceinline__ void load_u(const double* U, long long PS, const Geom& g, int x, int y,
-                                       int z, double& u1, double& u2, double& u3) {
-  bool fx = false, fy = false, fz = false;
-  const int xx = remap_axis(x, g.ax0, g.ax1, g.wall[0], g.wall[1], fx);
-  const int yy = remap_axis(y, g.ay0, g.ay1, g.wall[2], g.wall[3], fy);
-  const int zz = g.threed ? remap_axis(z, g.az0, g.az1, g.wall[4], g.wall[5], fz) : z;
-  const long long c = g.base + xx + (long long)yy * g.sy + (long long)zz * g.sz;
-  u1 = ldg<CG>(U + c);
-  u2 = ldg<CG>(U + PS + c);
-  u3 = ldg<CG>(U + 2 * PS + c);
-  if (fx) u1 = -u1;
-  if (fy) u2 = -u2;
-  if (fz) u3 = -u3;
-}
-
-// the gravitational acceleration at a cell: the donor's for a ghost coordinate,
-// reflected components negated like the momenta (the source update is exact
+// interior cells, or the gravitational acceleration (a ghost reads its donor's,
+// reflected components negated like the momenta: the source update is exact
 // under reflecting m and g together)
-__device__ __forceinline__ void load_g(const double* G, long long PS, const Geom& g, int x, int y,
-                                       int z, double& g1, double& g2, double& g3) {
-  load_u(G, PS, g, x, y, z, g1, g2, g3);
+template <bool CG = false>
+__device__ __forceinline__ void load_vec(const double* U, long long PS, const Place& p, double& u1,
+                                         double& u2, double& u3) {
+  const double* b = U + p.c;
+  u1 = ldg<CG>(b);
+  u2 = ldg<CG>(b + PS);
+  u3 = ldg<CG>(b + 2 * PS);
+  if (p.fx) u1 = -u1;
+  if (p.fy) u2 = -u2;
+  if (p.fz) u3 = -u3;
 }
 
 // source(0) with gravity on conserved values c (source.f90:161-182 with dt/2):
@@ -179,6 +179,7 @@ __device__ __forceinline__ void gravity_source0(Cons& c, double g1, double g2, d
 }
 
 __device__ __forceinline__ void apply_sources(Cons& c, int nsrc, double small_eps) {
+#pragma unroll 1
   for (int k = 0; k < nsrc; ++k) c.E = source_energy(c.d, c.m1, c.m2, c.m3, c.E, small_eps);
 }
 
@@ -209,16 +210,15 @@ __device__ __forceinline__ bool stage_is0(int rs) {
 }
 
 template <int STAGE, bool GRAV = false, bool CG = false>
-__device__ __forceinline__ Raw load_raw(const StageArgs& a, const Geom& g, int x, int y, int z,
-                                        int rs = 0) {
+__device__ __forceinline__ Raw load_raw(const StageArgs& a, const Place& p, int rs = 0) {
   const long long PS = a.ncells_total;
   Raw r;
   if (stage_is0<STAGE>(rs)) {
-    r.c = load_cons<CG>(a.X, PS, g, x, y, z);
-    if (GRAV) load_g(a.G, PS, g, x, y, z, r.v1, r.v2, r.v3);
+    r.c = load_cons<CG>(a.X, PS, p);
+    if (GRAV) load_vec<CG>(a.G, PS, p, r.v1, r.v2, r.v3);
   } else {
-    r.c = load_cons<CG>(a.Y, PS, g, x, y, z);
-    load_u<CG>(a.U, PS, g, x, y, z, r.v1, r.v2, r.v3);
+    r.c = load_cons<CG>(a.Y, PS, p);
+    load_vec<CG>(a.U, PS, p, r.v1, r.v2, r.v3);
   }
   return r;
 }
@@ -244,7 +244,8 @@ __device__ __forceinline__ bool prim_fast(const Geom& g, const Cons& c, double v
     const double kn = kHalf * (c.m1 * c.m1 + c.m2 * c.m2 + c.m3 * c.m3);
     ok = ok && quot_fast_ok(kn);
     const double ek = quot_fast(kn, d, r);
-    for (int k = 0; k < nsrc; ++k) E = fmax(E - ek, g.small_eps) + ek;
+#pragma unroll 1
+    for (int k = 0; k < nsrc; ++k) E = at_least(E - ek, g.small_eps) + ek;
   }
   ok = ok && quot_fast_ok(c.m1) && quot_fast_ok(c.m2) && quot_fast_ok(c.m3);
   q.d = d;
@@ -282,8 +283,8 @@ __device__ __forceinline__ Prim prim_ieee(double small_eps, double gm1, double g
 }
 
 template <int STAGE, bool GRAV = false, bool TAB = false, bool ANG = false>
-__device__ __forceinline__ Prim prim_of(const Geom& g, Raw r, unsigned& flags, int nsrc,
-                                        double dth, bool need_c = true, int rs = 0,
+__device__ __forceinline__ Prim prim_of(const Geom& g, Raw r, int nsrc, double dth,
+                                        bool need_c = true, int rs = 0,
                                         const EosDev* eos = nullptr) {
   Prim q;
   q.g = g.gam;
@@ -311,30 +312,16 @@ __device__ __forceinline__ Prim prim_of(const Geom& g, Raw r, unsigned& flags, i
     // eps; stage 1: the stage-0 velocity), then p and gamma by get_gamma2
     double eps = stage_is0<STAGE>(rs)
                      ? q.e
-                     : fmax(r.c.E - kin_rho_u(q.d, r.v1, r.v2, r.v3), g.small_eps);
+                     : at_least(r.c.E - kin_rho_u(q.d, r.v1, r.v2, r.v3), g.small_eps);
     double tk, m, gam;
     get_gamma2(*eos, eps, q.d, tk, m, gam);
     q.p = (q.d * tk * g.rgas / m);
     q.g = gam;
     q.c = need_c ? sqrt(q.p * gam / q.d) : 0.0;
   }
-  if (q.d < kLowRho) flags |= kFlagLowRho;
-  if (fabs(q.u1) > g.vlimit || fabs(q.u2) > g.vlimit || fabs(q.u3) > g.vlimit)
-    flags |= kFlagVlimit;
   return q;
 }
 
-// Primitives seen by flux(avg) at a cell.
-//  stage 0: cons = src^nsrc(X); u = m/rho (velocity at main.f90:318); p from
-//           state() with the velocity array of the previous step, which equals
-//           m/rho of the same momenta (source adds zero momentum).
-//  stage 1: cons = Y; u = m/rho of Y (velocity at main.f90:355); p from state()
-//           with the stage-0 velocity m0/rho0 (main.f90:353 uses the stale u),
-//           which stage 0 stored in U (the same quotient, so the same bits).
-//  GRAV (a gravitational force this step): stage 0 takes the nsrc-1 force-free
-//           sources still pending, then source(0) with the force, which kicks
-//           the momenta; state() then reads the velocity array of before the
-//           kick (main.f90:318-319 call state() before velocity()).
 // the centre of cell (ix, iy) in the x-y plane (flux_ang.f90:44-46 and
 // :571-573, as cell_xy), and its distance from the z axis
 __device__ __forceinline__ void cell_xyr(const Geom& g, int ix, int iy, double& x, double& y,
@@ -354,18 +341,6 @@ __device__ __forceinline__ void ang_to(const Geom& g, int ix, int iy, double m1,
   r = sqrt(x * x + y * y);
   rm = (m1 * x + m2 * y) / r;
   am = x * m2 - y * m1;
-}
-
-template <int STAGE, bool GRAV = false, bool CG = false, bool TAB = false, bool ANG = false>
-__device__ __forceinline__ Prim load_prim(const StageArgs& a, const Geom& g, int x, int y, int z,
-                                          unsigned& flags, int nsrc, double dth,
-                                          bool need_c = true, int rs = 0) {
-  const Raw r = load_raw<STAGE, GRAV, CG>(a, g, x, y, z, rs);
-  Prim q = prim_of<STAGE, GRAV, TAB, ANG>(g, r, flags, nsrc, dth, need_c, rs, &a.eos);
-  // with flux_ang the momenta reconstructed are the transformed ones (the
-  // sources leave the momenta alone)
-  if (ANG) ang_to(g, x, y, r.c.m1, r.c.m2, q.rm, q.am);
-  return q;
 }
 
 template <bool POW2, bool TAB = false, bool ANG = false>
@@ -416,6 +391,15 @@ __device__ __forceinline__ Prim get_prim(const double* SP, int i) {
     q.rm = SP[7 * NP + i];
     q.am = SP[8 * NP + i];
   }
+  return q;
+}
+// the primitives of cell i with the velocities along (u1) and across (u2) the
+// axis ax = 0 (x) or 1 (y) of the face states to be formed
+template <int NP, int NPF = 7>
+__device__ __forceinline__ Prim get_prim_along(const double* SP, int i, int ax) {
+  Prim q = get_prim<NP, NPF>(SP, i);
+  q.u1 = SP[(1 + ax) * NP + i];
+  q.u2 = SP[(2 - ax) * NP + i];
   return q;
 }
 template <int NSF = 6>
@@ -475,7 +459,7 @@ __device__ __forceinline__ bool epi_fast(const Geom& g, const double n[5], doubl
   u2 = quot_fast(n[2], d, r);
   u3 = quot_fast(n[3], d, r);
   const double ek = quot_fast(kn, d, r);
-  const double E3 = fmax(n[4] - ek, g.small_eps) + ek;
+  const double E3 = at_least(n[4] - ek, g.small_eps) + ek;
   const double pA = eos_pressure(d, E3, u1, u2, u3, g.gm1, g.small_eps);
   const double pn = g.gam * pA;
   ok = ok && rad_fast_ok(pn);
@@ -508,7 +492,7 @@ __device__ __forceinline__ void epi_tab(const Geom& g, const EosDev& eos, const 
   u2 = n[2] / n[0];
   u3 = n[3] / n[0];
   const double E3 = source_energy(n[0], n[1], n[2], n[3], n[4], g.small_eps);
-  double eps = fmax(E3 - kin_rho_u(n[0], u1, u2, u3), g.small_eps);
+  double eps = at_least(E3 - kin_rho_u(n[0], u1, u2, u3), g.small_eps);
   double tk, m, gam;
   get_gamma2(eos, eps, n[0], tk, m, gam);
   const double p = (n[0] * tk * g.rgas / m);
@@ -516,12 +500,42 @@ __device__ __forceinline__ void epi_tab(const Geom& g, const EosDev& eos, const 
 }
 
 // ------------------------------------------------------------------ stage kernel
-// One tile of one stage.  FULL: the tile is a whole TX x TY block of interior
-// columns, so its extents are compile-time constants.
+// One tile of one stage: TX x TY columns marched along z.  Per plane:
+//  A  primitives of the tile's cells and its two-cell x/y halo to shared memory
+//     (own cells from the z pipeline, which is loaded two planes ahead; halo
+//     cells computed here, at most one a thread), all loads before the arithmetic
+//  B  the minus and plus face states in x and y of every cell next to a face
+//  C  every x and y face flux once
+//  D  the z states two cells up the own column, the z face above the own cell,
+//     and the own cell's update.
+// B and C run both axes through one code, with the velocities along and across
+// the axis in each other's place for y (the HLL flux is the same arithmetic with
+// them exchanged); what an item of a thread reads is worked out once per tile and
+// kept in a table (s_item), not per plane.  A plane takes three barriers: the
+// fluxes go where the states they came from were, so nothing of D is overwritten
+// by A of the next plane.
+//
+// What bounds it (ncu, 128^3, stage 0 / 1): not memory (DRAM 8-12 % busy) but the
+// latency of the FP64 chains at 16 warps per SM, the registers' limit: 53 / 52 %
+// of issue slots, 45 % of the FP64 pipe; of 7.1 warp cycles per instruction 1.65
+// wait on a fixed latency, 1.2 at a barrier, 0.5 for the FP64 pipe, 0.6-0.8 for
+// global loads.  So the gains lie in fewer instructions and no spills.  Measured
+// per 256^3 step on one box: 4.68 ms with a code path per axis, every bound by
+// fmax and fluxes over the primitives (a fourth barrier); 4.64 with both axes in
+// one path and compare-and-select bounds (2420 and 2690 executed instructions per
+// cell); 4.20 with the item table, the places of own and halo cells worked out
+// once per tile (2240 and 2400) and the fluxes' dividing code once; 4.11 with three
+// barriers.  The halo cell's loads are issued after the own cell's arithmetic:
+// both at once spill 84-124 bytes per thread and measured 4.57 ms.  A rim warp
+// that takes all halo work, with states and fluxes passed by shuffles, measured
+// 5.7 ms (its chain of five primitives paces the block, and 140-190 KB of code
+// against 60 miss in the instruction cache).
 // dt: the step's full dt; nsrc: the sources the stage input is short of (both
 // read from the box's control block by the caller).  CG: inputs through L2 (the
 // persistent batched kernel).
-template <class S, int STAGE, bool POW2, bool THREED, bool FULL, bool GRAV, bool CG = false>
+enum : unsigned { kItemY = 1u << 12, kItemGhost = 1u << 13, kItemIn = 1u << 14 };
+
+template <class S, int STAGE, bool POW2, bool THREED, bool GRAV, bool CG = false>
 __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, const Geom& g,
                                            Ctrl* C, double dt, int nsrc, double* sm,
                                            double* red_rate, unsigned* red_flags, int rs = 0) {
@@ -529,351 +543,340 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
   constexpr int TX = S::TX, TY = S::TY, NT = S::NT, PW = S::PW, NP = S::NP;
   constexpr bool TAB = S::TAB, ANG = S::ANG;
   constexpr int NPF = S::NPF, NSF = S::NSF, NFQ = S::NFQ, NOWN = S::NOWN;
-  constexpr int NSX = S::NSX, NSY = S::NSY, NFX = S::NFX, NFY = S::NFY, NR0 = S::NR0;
-  double* SP = sm;                    // [NPF][TY+4][TX+4] primitives of the plane
-  double* SX = sm + NR0;              // [2 NSF][TY][TX+2] x states (minus, then plus)
-  double* SY = SX + 2 * NSF * NSX;    // [2 NSF][TY+2][TX] y states
-  double* FX = sm;                    // [NFQ][TY][TX+1] x face fluxes (aliases SP)
-  double* FY = sm + NFQ * NFX;        // [NFQ][TY+1][TX] y face fluxes
-  double* ZS = SY + 2 * NSF * NSY;    // [10 + NSF][NOWN]: Fzm 0-4, Fzp 5-9, plus state 10-
+  constexpr int NSX = S::NSX, NS = S::NSX + S::NSY, NFX = S::NFX, NF = S::NFX + S::NFY;
+  double* SP = sm;                  // [NPF][TY+4][TX+4] primitives of the plane
+  double* SS = sm + NPF * NP;       // [2 NSF] minus, then plus: x [TY][TX+2], y [TY+2][TX]
+  // face fluxes: each state is read by one face only, so a face's flux takes the
+  // place of the plus state below it
+  double* FF = SS + NSF * NS;
+  double* ZS = SS + 2 * NSF * NS;   // [10 + NSF][NOWN]: z flux, its difference over the plane, plus z state
+  unsigned short* s_item = reinterpret_cast<unsigned short*>(ZS + (10 + NSF) * NOWN);  // [NS]
   const double dth = dt * kHalf;  // the sources' half step (main.f90:282,471)
 
   const int tid = threadIdx.x;
   const int tx = tid % TX, ty = tid / TX;
-  const int NAx = g.ax1 - g.ax0, NAy = g.ay1 - g.ay0;
-  const int w = FULL ? TX : min(TX, NAx - t.x0), h = FULL ? TY : min(TY, NAy - t.y0);
+  const int w = min(TX, g.ax1 - g.ax0 - t.x0), h = min(TY, g.ay1 - g.ay0 - t.y0);
   const bool own = (tx < w) && (ty < h);
   const int bx0 = g.ax0 + t.x0, by0 = g.ay0 + t.y0;  // full-grid tile origin
   const int gx = bx0 + tx, gy = by0 + ty;
-  const int nhalo = 4 * h + 4 * w;
-  const int nxs = (w + 2) * h, nys = w * (h + 2);
-  const int nxf = (w + 1) * h, nyf = w * (h + 1);
+  const int z0 = g.az0 + t.z0, z1 = g.az0 + t.z1;
   const long long PS = a.ncells_total;
-  const double idz = g.idz;
 
   unsigned flags = 0;
   double rate = 0.0;
 
-  // z pipeline of the own column (3-D grids)
-  Prim Pk, Pk1;
-  // (columns only: the threads with a column are 0 .. NOWN-1)
-  auto zs = [&](int k) -> double& { return ZS[k * NOWN + threadIdx.x]; };
-
-  const int z0 = g.az0 + t.z0, z1 = g.az0 + t.z1;
-  if (THREED && own) {
-    const Prim Pm2 = load_prim<STAGE, GRAV, CG, TAB, ANG>(a, g, gx, gy, z0 - 2, flags, nsrc, dth, true, rs);
-    const Prim Pm1 = load_prim<STAGE, GRAV, CG, TAB, ANG>(a, g, gx, gy, z0 - 1, flags, nsrc, dth, true, rs);
-    Pk = load_prim<STAGE, GRAV, CG, TAB, ANG>(a, g, gx, gy, z0, flags, nsrc, dth, true, rs);
-    Pk1 = load_prim<STAGE, GRAV, CG, TAB, ANG>(a, g, gx, gy, z0 + 1, flags, nsrc, dth, true, rs);
-    FaceState mm, pm, m0;
-    if (z0 - 1 < g.az0) {
-      ghost_states(Pm1, mm, pm);
-    } else {
-      dir_states<POW2, TAB, ANG>(Pm2, Pm1, Pk, Pm1.u3, dt, g.dz, idz, mm, pm);
-    }
-    FaceState plusk;
-    double Fzm[5];
-    dir_states<POW2, TAB, ANG>(Pm1, Pk, Pk1, Pk.u3, dt, g.dz, idz, m0, plusk);
-    if (ANG) {
-      double F7[7];
-      hll_flux_ang<2>(pm, m0, g.gam, 0.0, 0.0, 1.0, 0.0, 0.0, 1.0, F7);
-      for (int q = 0; q < 5; ++q) Fzm[q] = F7[q];
-    } else {
-      hll_flux<2, TAB>(pm, m0, g.gam, Fzm);
-    }
-    for (int q = 0; q < 5; ++q) zs(q) = Fzm[q];
-    zs(10) = plusk.d; zs(11) = plusk.u1; zs(12) = plusk.u2; zs(13) = plusk.u3;
-    zs(14) = plusk.p; zs(15) = plusk.e;
-    if (TAB) zs(16) = plusk.g;
-    if (ANG) { zs(16) = plusk.rm; zs(17) = plusk.am; }
+  // the table of state items: the cell in SP
+  for (int i = tid; i < NS; i += NT) {
+    const int ax = i >= NSX, k = i - NSX;
+    const int cy = ax ? k / TX - 1 : i / (TX + 2), cx = ax ? k % TX : i % (TX + 2) - 1;
+    const int f = ax ? by0 + cy : bx0 + cx;
+    const bool ghost = f < (ax ? g.ay0 : g.ax0) || f >= (ax ? g.ay1 : g.ax1);
+    s_item[i] = (unsigned short)(((cy + 2) * PW + cx + 2) | (ax ? kItemY : 0u) |
+                                 (ghost ? kItemGhost : 0u) |
+                                 (cx < w + 1 - ax && cy < h + ax ? kItemIn : 0u));
   }
 
-  for (int z = (THREED ? z0 : g.az0 + t.z0); z < (THREED ? z1 : g.az0 + t.z1); ++z) {
-    // ---- A: primitives of plane z (own from the pipeline, halo computed here)
-    if (!is0 && own) {
-      // the update at the end of this plane reads the step input of the own
-      // cell, which nothing in this stage loaded before: start it towards L2
-      const double* c = a.X + g.base + gx + (long long)gy * g.sy + (long long)z * g.sz;
-#pragma unroll
-      for (int q = 0; q < 5; ++q) asm volatile("prefetch.global.L2 [%0];" ::"l"(c + q * PS));
-      if (THREED && z + 3 < g.az1) {
-        // the own column's loads of the next plane iteration
-        const long long o3 = g.base + gx + (long long)gy * g.sy + (long long)(z + 3) * g.sz;
-#pragma unroll
-        for (int q = 0; q < 5; ++q) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.Y + o3 + q * PS));
-#pragma unroll
-        for (int q = 0; q < 3; ++q) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.U + o3 + q * PS));
-      }
+  // the halo cell of this thread (those without a column first), if any
+  static_assert(4 * (TX + TY) <= NT, "one halo cell per thread and plane at most");
+  Place hp{0, false, false, false};
+  int hc = -1;  // its place in SP
+  {
+    const int i = (tid + NT - NOWN) % NT;
+    int cx, cy;
+    bool in;
+    if (i < 4 * TY) {
+      const int j = i & 3;
+      cy = i >> 2;
+      cx = j < 2 ? j - 2 : w + j - 2;
+      in = cy < h;
+    } else {
+      const int k = i - 4 * TY, j = k / TX;
+      cx = k % TX;
+      cy = j < 2 ? j - 2 : h + j - 2;
+      in = j < 4 && cx < w;
     }
-    if (is0 && own && THREED && z + 3 < g.az1) {
-      // stage 0: the own column's step input of the next plane iteration
-      const long long o3 = g.base + gx + (long long)gy * g.sy + (long long)(z + 3) * g.sz;
-#pragma unroll
-      for (int q = 0; q < 5; ++q) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.X + o3 + q * PS));
+    if (in) {
+      hp = place_of(g, bx0 + cx, by0 + cy, g.az0);
+      hp.c -= (long long)g.az0 * g.sz;
+      hc = (cy + 2) * PW + cx + 2;
     }
+  }
+  const long long co = g.base + gx + (long long)gy * g.sy;  // the own column
+  auto zs = [&](int k) -> double& { return ZS[k * NOWN + tid]; };
+  auto own_place = [&](int z) {
+    Place p{0, false, false, false};
+    const int zz = THREED ? remap_axis(z, g.az0, g.az1, g.wall[4], g.wall[5], p.fz) : z;
+    p.c = co + (long long)zz * g.sz;
+    return p;
+  };
+  auto prim_at = [&](const Raw& r, int x, int y) {
+    Prim q = prim_of<STAGE, GRAV, TAB, ANG>(g, r, nsrc, dth, true, rs, &a.eos);
+    // with flux_ang the momenta reconstructed are the transformed ones (the
+    // sources leave the momenta alone)
+    if (ANG) ang_to(g, x, y, r.c.m1, r.c.m2, q.rm, q.am);
+    return q;
+  };
+
+  // z pipeline of the own column (3-D grids): primitives of planes z and z+1
+  Prim Pk, Pk1;
+  if (THREED && own) {
+    const Raw r0 = load_raw<STAGE, GRAV, CG>(a, own_place(z0 - 2), rs);
+    const Raw r1 = load_raw<STAGE, GRAV, CG>(a, own_place(z0 - 1), rs);
+    Pk = prim_at(r0, gx, gy);
+    Pk1 = prim_at(r1, gx, gy);
+  }
+
+  // in 3-D the first two rounds only fill the z pipeline
+  for (int z = THREED ? z0 - 2 : z0; z < z1; ++z) {
+    const bool plane = !THREED || z >= z0;
+    const long long o = co + (long long)z * g.sz;  // the own cell
+    // ---- A
     Prim P2;
-    FaceState mz1, pz1;
-    if (own) {
-      if (THREED) {
-        P2 = load_prim<STAGE, GRAV, CG, TAB, ANG>(a, g, gx, gy, z + 2, flags, nsrc, dth, true, rs);
-      } else {
-        Pk = load_prim<STAGE, GRAV, CG, TAB, ANG>(a, g, gx, gy, z, flags, nsrc, dth, true, rs);
+    {
+      Raw ro, rh;
+      const bool halo = plane && hc >= 0;
+      if (own) ro = load_raw<STAGE, GRAV, CG>(a, own_place(THREED ? z + 2 : z), rs);
+      if (own) {
+        // towards L2: the step input that stage 1's update reads at the end of
+        // this plane, and the own column's loads of the next plane
+        if (!is0 && plane) {
+#pragma unroll
+          for (int q = 0; q < 5; ++q) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.X + o + q * PS));
+        }
+        if (THREED && z + 3 < g.az1) {
+          const long long o3 = o + 3 * g.sz;
+          const double* B = is0 ? a.X : a.Y;
+#pragma unroll
+          for (int q = 0; q < 5; ++q) asm volatile("prefetch.global.L2 [%0];" ::"l"(B + o3 + q * PS));
+          if (!is0) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.U + o3 + q * PS));
+          }
+        }
+        if (THREED) P2 = prim_at(ro, gx, gy);
+        else Pk = prim_at(ro, gx, gy);
+        if (plane) {
+          put_prim<NP, NPF>(SP, (ty + 2) * PW + tx + 2, Pk);
+          // the guards look at every interior cell where it is an own cell
+          if (Pk.d < kLowRho) flags |= kFlagLowRho;
+          if (fabs(Pk.u1) > g.vlimit || fabs(Pk.u2) > g.vlimit || fabs(Pk.u3) > g.vlimit)
+            flags |= kFlagVlimit;
+          if (is0) {
+            // sources change only E, so this is m/rho of the step input
+            a.U[o] = Pk.u1;
+            a.U[PS + o] = Pk.u2;
+            a.U[2 * PS + o] = Pk.u3;
+          }
+        }
       }
-      put_prim<NP, NPF>(SP, (ty + 2) * PW + (tx + 2), Pk);
-      if (is0) {
-        // sources change only E, so this is m/rho of the step input
-        const long long o = g.base + gx + (long long)gy * g.sy + (long long)z * g.sz;
-        a.U[o] = Pk.u1;
-        a.U[PS + o] = Pk.u2;
-        a.U[2 * PS + o] = Pk.u3;
-      }
-    }
-    // halo cells go first to the threads without a column of their own (at most
-    // one per thread: 4*(TX+TY) <= NT).  Their loads are not issued before the
-    // own column's arithmetic: holding both cells' values at once spills
-    // registers and measured 14 % slower.
-    for (int i = (tid + NT - TX * TY) % NT; i < nhalo; i += NT) {
-      int cx, cy;
-      if (i < 4 * h) {
-        cy = i >> 2;
-        const int j = i & 3;
-        cx = j < 2 ? j - 2 : w + (j - 2);
-      } else {
-        const int k = i - 4 * h;
-        cx = k % w;
-        const int j = k / w;
-        cy = j < 2 ? j - 2 : h + (j - 2);
-      }
-      // cells two away from the tile only feed slopes; ghost cells need no lambda
-      const int fx = bx0 + cx, fy = by0 + cy;
-      const bool near = cx >= -1 && cx <= w && cy >= -1 && cy <= h;
-      const bool inner = fx >= g.ax0 && fx < g.ax1 && fy >= g.ay0 && fy < g.ay1;
-      const Prim q = load_prim<STAGE, GRAV, CG, TAB, ANG>(a, g, fx, fy, z, flags, nsrc, dth, near && inner, rs);
-      put_prim<NP, NPF>(SP, (cy + 2) * PW + (cx + 2), q);
-    }
-    if (THREED && own) {
-      if (z + 1 >= g.az1) {
-        ghost_states(Pk1, mz1, pz1);
-      } else {
-        dir_states<POW2, TAB, ANG>(Pk, Pk1, P2, Pk1.u3, dt, g.dz, idz, mz1, pz1);
-      }
-      const FaceState plusk{zs(10), zs(11), zs(12), zs(13), zs(14), zs(15),
-                            TAB ? zs(16) : 0.0,
-                            ANG ? zs(16) : 0.0, ANG ? zs(17) : 0.0};
-      double Fzp[5];
-      if (ANG) {
-        double F7[7];
-        hll_flux_ang<2>(plusk, mz1, g.gam, 0.0, 0.0, 1.0, 0.0, 0.0, 1.0, F7);
-        for (int q = 0; q < 5; ++q) Fzp[q] = F7[q];
-      } else {
-        hll_flux<2, TAB>(plusk, mz1, g.gam, Fzp);
-      }
-      for (int q = 0; q < 5; ++q) zs(5 + q) = Fzp[q];
-      zs(10) = pz1.d; zs(11) = pz1.u1; zs(12) = pz1.u2; zs(13) = pz1.u3;
-      zs(14) = pz1.p; zs(15) = pz1.e;
-      if (TAB) zs(16) = pz1.g;
-      if (ANG) { zs(16) = pz1.rm; zs(17) = pz1.am; }
-    }
-    __syncthreads();
+      if (halo) {
+        Place p = hp;
+        p.c += (long long)z * g.sz;
+        rh = load_raw<STAGE, GRAV, CG>(a, p, rs);
 
-    // ---- B: x and y face states of the plane.  The y items start at a warp
-    // boundary, so no warp runs both the x and the y code (the x items end in
-    // idle lanes instead)
-    const int nxs_w = (nxs + 31) & ~31;
-    for (int i = tid; i < nxs_w + nys; i += NT) {
-      FaceState mi, pl;
-      if (i < nxs_w) {
-        if (i >= nxs) continue;
-        const int cy = i / (w + 2), cx = i % (w + 2) - 1;
-        const int c = (cy + 2) * PW + (cx + 2);
-        const Prim q = get_prim<NP, NPF>(SP, c);
-        const int fx = bx0 + cx;
-        if (fx < g.ax0 || fx >= g.ax1) {
+        const int cy = hc / PW - 2, cx = hc % PW - 2;
+        put_prim<NP, NPF>(SP, hc, prim_at(rh, bx0 + cx, by0 + cy));
+      }
+      // the z states of the cell above and the z face between
+      if (THREED && own) {
+        FaceState mz, pz;
+        if (z + 1 < g.az0 || z + 1 >= g.az1) {
+          ghost_states(Pk1, mz, pz);
+        } else {
+          dir_states<POW2, TAB, ANG>(Pk, Pk1, P2, Pk1.u3, dt, g.dz, g.idz, mz, pz);
+        }
+        Pk = Pk1;
+        Pk1 = P2;
+        if (z >= z0 - 1) {
+          const FaceState plusk = get_fs<NSF>(ZS + 10 * NOWN, NOWN, tid);
+          double Fz[5];
+          if (ANG) {
+            double F7[7];
+            hll_flux_ang<2>(plusk, mz, g.gam, 0.0, 0.0, 1.0, 0.0, 0.0, 1.0, F7);
+            for (int q = 0; q < 5; ++q) Fz[q] = F7[q];
+          } else {
+            hll_flux<2, TAB>(plusk, mz, g.gam, Fz);
+          }
+  #pragma unroll
+          for (int q = 0; q < 5; ++q) {
+            zs(5 + q) = Fz[q] - zs(q);
+            zs(q) = Fz[q];
+          }
+        }
+        put_fs<NSF>(ZS + 10 * NOWN, NOWN, tid, pz);
+      }
+    }
+    if (plane) {
+      __syncthreads();
+      // ---- B: x and y face states of the plane
+      for (int i = tid; i < NS; i += NT) {
+        const unsigned e = s_item[i];
+        if (!(e & kItemIn)) continue;
+        const int ax = (e & kItemY) ? 1 : 0, c = e & 0xfffu, st = ax ? PW : 1;
+        const Prim q = get_prim_along<NP, NPF>(SP, c, ax);
+        FaceState mi, pl;
+        if (e & kItemGhost) {
           ghost_states(q, mi, pl);
         } else {
-          dir_states<POW2, TAB, ANG>(get_prim<NP, NPF>(SP, c - 1), q, get_prim<NP, NPF>(SP, c + 1), q.u1, dt, g.dx, g.idx, mi,
-                           pl);
+          dir_states<POW2, TAB, ANG>(get_prim_along<NP, NPF>(SP, c - st, ax), q,
+                                     get_prim_along<NP, NPF>(SP, c + st, ax), q.u1, dt,
+                                     ax ? g.dy : g.dx, ax ? g.idy : g.idx, mi, pl);
         }
-        const int o = cy * (TX + 2) + (cx + 1);
-        put_fs<NSF>(SX, NSX, o, mi);
-        put_fs<NSF>(SX + NSF * NSX, NSX, o, pl);
-      } else {
-        const int k = i - nxs_w;
-        const int cy = k / w - 1, cx = k % w;
-        const int c = (cy + 2) * PW + (cx + 2);
-        const Prim q = get_prim<NP, NPF>(SP, c);
-        const int fy = by0 + cy;
-        if (fy < g.ay0 || fy >= g.ay1) {
-          ghost_states(q, mi, pl);
-        } else {
-          dir_states<POW2, TAB, ANG>(get_prim<NP, NPF>(SP, c - PW), q, get_prim<NP, NPF>(SP, c + PW), q.u2, dt, g.dy, g.idy,
-                           mi, pl);
-        }
-        const int o = (cy + 1) * TX + cx;
-        put_fs<NSF>(SY, NSY, o, mi);
-        put_fs<NSF>(SY + NSF * NSY, NSY, o, pl);
+        put_fs<NSF>(SS, NS, i, mi);
+        put_fs<NSF>(FF, NS, i, pl);
       }
-    }
-    __syncthreads();
-
-    // ---- C: x and y face fluxes (face f lies between cells f-1 and f); the y
-    // faces start at a warp boundary as in B
-    const int nxf_w = (nxf + 31) & ~31;
-    for (int i = tid; i < nxf_w + nyf; i += NT) {
-      double F[NFQ];
-      if (i < nxf_w) {
-        if (i >= nxf) continue;
-        const int cy = i / (w + 1), f = i % (w + 1);
-        const int base = cy * (TX + 2);
-        const FaceState L = get_fs<NSF>(SX + NSF * NSX, NSX, base + f);  // plus state of cell f-1
-        const FaceState R = get_fs<NSF>(SX, NSX, base + f + 1);        // minus state of cell f
+      __syncthreads();
+      // ---- C: x and y face fluxes (face f lies between cells f-1 and f)
+      for (int i = tid; i < NF; i += NT) {
+        const int ax = i >= NFX, k = i - NFX;
+        const int cy = ax ? k / TX : i / (TX + 1), cx = ax ? k % TX : i % (TX + 1);
+        if (cx >= w + 1 - ax || cy >= h + ax) continue;
+        const int lo = ax ? NSX + k : i + cy;
+        // the plus state of the cell below the face and the minus state of the one above
+        const FaceState L = get_fs<NSF>(FF, NS, lo);
+        const FaceState R = get_fs<NSF>(SS, NS, lo + (ax ? TX : 1));
+        double F[NFQ];
         if constexpr (ANG) {
           // the momentum fluxes for both cells of the face (their own centres)
           double xl, yl, rl, xh, yh, rh;
-          cell_xyr(g, bx0 + f - 1, by0 + cy, xl, yl, rl);
-          cell_xyr(g, bx0 + f, by0 + cy, xh, yh, rh);
-          hll_flux_ang<0>(L, R, g.gam, xl, yl, rl, xh, yh, rh, F);
+          cell_xyr(g, bx0 + cx - 1 + ax, by0 + cy - ax, xl, yl, rl);
+          cell_xyr(g, bx0 + cx, by0 + cy, xh, yh, rh);
+          if (ax) {
+            FaceState l = L, r = R;
+            l.u1 = L.u2; l.u2 = L.u1; r.u1 = R.u2; r.u2 = R.u1;
+            hll_flux_ang<1>(l, r, g.gam, xl, yl, rl, xh, yh, rh, F);
+          } else {
+            hll_flux_ang<0>(L, R, g.gam, xl, yl, rl, xh, yh, rh, F);
+          }
+#pragma unroll
+          for (int q = 0; q < NFQ; ++q) FF[q * NS + lo] = F[q];
         } else {
           hll_flux<0, TAB>(L, R, g.gam, F);
+          FF[lo] = F[0];
+          FF[(1 + ax) * NS + lo] = F[1];
+          FF[(2 - ax) * NS + lo] = F[2];
+          FF[3 * NS + lo] = F[3];
+          FF[4 * NS + lo] = F[4];
         }
-        const int o = cy * (TX + 1) + f;
-#pragma unroll
-        for (int q = 0; q < NFQ; ++q) FX[q * NFX + o] = F[q];
-      } else {
-        const int k = i - nxf_w;
-        const int f = k / w, cx = k % w;
-        const FaceState L = get_fs<NSF>(SY + NSF * NSY, NSY, f * TX + cx);
-        const FaceState R = get_fs<NSF>(SY, NSY, (f + 1) * TX + cx);
-        if constexpr (ANG) {
-          double xl, yl, rl, xh, yh, rh;
-          cell_xyr(g, bx0 + cx, by0 + f - 1, xl, yl, rl);
-          cell_xyr(g, bx0 + cx, by0 + f, xh, yh, rh);
-          hll_flux_ang<1>(L, R, g.gam, xl, yl, rl, xh, yh, rh, F);
-        } else {
-          hll_flux<1, TAB>(L, R, g.gam, F);
-        }
-        const int o = f * TX + cx;
-#pragma unroll
-        for (int q = 0; q < NFQ; ++q) FY[q * NFY + o] = F[q];
       }
+      __syncthreads();
     }
-    __syncthreads();
 
-    // ---- D: conservative update of the own cell (flux.f90:186-230)
+    // ---- D: the z face above the own cell, and its update (flux.f90:186-230)
     if (own) {
-      double ft[5];
-#pragma unroll
-      for (int q = 0; q < 5; ++q) {
-        // with flux_ang the momentum fluxes of this cell's plus faces are the
-        // versions for their low cell (planes 5, 6)
-        const int qp = (ANG && (q == 1 || q == 2)) ? q + 4 : q;
-        const double dfx = FX[qp * NFX + ty * (TX + 1) + tx + 1] - FX[q * NFX + ty * (TX + 1) + tx];
-        const double dfy = FY[qp * NFY + (ty + 1) * TX + tx] - FY[q * NFY + ty * TX + tx];
-        double sum = g.ayz * dfx + g.axz * dfy;
-        if (THREED) sum = sum + g.axy * (zs(5 + q) - zs(q));
-        ft[q] = POW2 ? -sum * dt * g.ivol : cdiv(-sum * dt, g.vol, g.ivol);
-      }
-      Cons c0 = load_cons<CG>(a.X, PS, g, gx, gy, z);
+      Cons c0, c1;
       double go1 = 0.0, go2 = 0.0, go3 = 0.0;  // the own cell's acceleration
-      if (GRAV) {
-        load_g(a.G, PS, g, gx, gy, z, go1, go2, go3);
-        double v1, v2, v3;
-        apply_sources(c0, nsrc - 1, g.small_eps);
-        gravity_source0(c0, go1, go2, go3, dth, g.small_eps, v1, v2, v3);
-      } else {
-        const SharedDiv q0(c0.d);
-        for (int k = 0; k < nsrc; ++k)
-          c0.E = source_energy_q(q0, c0.m1, c0.m2, c0.m3, c0.E, g.small_eps);
+      if (plane) {
+        const Place p{o, false, false, false};
+        c0 = load_cons<CG>(a.X, PS, p);
+        if (!is0) c1 = load_cons<CG>(a.Y, PS, p);
+        if (GRAV) load_vec<CG>(a.G, PS, p, go1, go2, go3);
       }
-      double n[5];
-      // flux_ang updates the transformed momenta (flux_ang.f90:44-62, 149-246)
-      if (ANG) ang_to(g, gx, gy, c0.m1, c0.m2, c0.m1, c0.m2);
-      if (is0) {
-        n[0] = c0.d + ft[0];
-        n[1] = c0.m1 + ft[1];
-        n[2] = c0.m2 + ft[2];
-        n[3] = c0.m3 + ft[3];
-        n[4] = c0.E + ft[4];
-      } else {
-        Cons c1 = load_cons<CG>(a.Y, PS, g, gx, gy, z);
-        if (ANG) ang_to(g, gx, gy, c1.m1, c1.m2, c1.m1, c1.m2);
-        n[0] = kHalf * (c0.d + c1.d + ft[0]);
-        n[1] = kHalf * (c0.m1 + c1.m1 + ft[1]);
-        n[2] = kHalf * (c0.m2 + c1.m2 + ft[2]);
-        n[3] = kHalf * (c0.m3 + c1.m3 + ft[3]);
-        n[4] = kHalf * (c0.E + c1.E + ft[4]);
-      }
-      if (ANG) {
-        // back to (m1, m2) (flux_ang.f90:247-270)
-        double cxp, cyp, crp;
-        cell_xyr(g, gx, gy, cxp, cyp, crp);
-        const double tyy = cyp + g.yoff, trr = sqrt(cxp * cxp + tyy * tyy);
-        const double rmom = n[1], angmom = n[2];
-        n[1] = (rmom * cxp - angmom * tyy / trr) / trr;
-        n[2] = (rmom * tyy + angmom * cxp / trr) / trr;
-      }
-      floors(n[0], n[1], n[2], n[3], n[4], g.small_rho, g.small_eps);
-      if (!(isfinite(n[0]) && isfinite(n[1]) && isfinite(n[2]) && isfinite(n[3]) &&
-            isfinite(n[4])))
-        flags |= kFlagNonFinite;
-      if (!is0) {
-        // state/velocity after flux(1) and after source(1) (main.f90:372-380,490-515);
-        // without a force every division here is by the new density: one
-        // reciprocal and one window check for all of them (epi_fast)
-        double u1, u2, u3, r0 = 0.0;
-        if (GRAV) {
-          const SharedDiv qn(n[0]);
-          u1 = qn(n[1]);
-          u2 = qn(n[2]);
-          u3 = qn(n[3]);
-        } else if (TAB) {
-          epi_tab<POW2>(g, a.eos, n, u1, u2, u3, r0);
-        } else if (!epi_fast<POW2>(g, n, u1, u2, u3, r0)) {
-          epi_ieee<POW2>(g, n, u1, u2, u3, r0);
+      if (plane) {
+        double ft[5];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+          // with flux_ang the momentum fluxes of this cell's plus faces are the
+          // versions for their low cell (planes 5, 6)
+          const int qp = (ANG && (q == 1 || q == 2)) ? q + 4 : q;
+          const int fx = ty * (TX + 2) + tx, fy = NSX + ty * TX + tx;
+          const double dfx = FF[qp * NS + fx + 1] - FF[q * NS + fx];
+          const double dfy = FF[qp * NS + fy + TX] - FF[q * NS + fy];
+          double sum = g.ayz * dfx + g.axz * dfy;
+          if (THREED) sum = sum + g.axy * zs(5 + q);
+          ft[q] = POW2 ? -sum * dt * g.ivol : cdiv(-sum * dt, g.vol, g.ivol);
         }
-        if (n[0] < kLowRho) flags |= kFlagLowRho;
-        if (fabs(u1) > g.vlimit || fabs(u2) > g.vlimit || fabs(u3) > g.vlimit)
-          flags |= kFlagVlimit;
         if (GRAV) {
-          // source(1) with the force (main.f90:471): the planes take its result,
-          // the velocity it read goes to UC for state() at the step's end
-          // (main.f90:513-514), and the Courant rate of the next step is taken
-          // with the velocity after it (main.f90:515)
-          const long long o = g.base + gx + (long long)gy * g.sy + (long long)z * g.sz;
-          a.UC[o] = u1;
-          a.UC[PS + o] = u2;
-          a.UC[2 * PS + o] = u3;
-          source_gravity(n[0], n[1], n[2], n[3], n[4], go1, go2, go3, u1, u2, u3, dth,
-                         g.small_eps);
-          const double w1 = n[1] / n[0], w2 = n[2] / n[0], w3 = n[3] / n[0];
-          if (fabs(w1) > g.vlimit || fabs(w2) > g.vlimit || fabs(w3) > g.vlimit)
-            flags |= kFlagVlimit;
-          if (!(isfinite(n[1]) && isfinite(n[2]) && isfinite(n[3]) && isfinite(n[4])))
-            flags |= kFlagNonFinite;
-          const double pA = eos_pressure(n[0], n[4], w1, w2, w3, g.gm1, g.small_eps);
-          const double r0 = courant_rate<POW2>(n[0], pA, g.gam, w1, w2, w3, g.dx, g.dy, g.dz,
-                                               g.idx, g.idy, g.idz);
-          rate = fmax(rate, r0);
-          if (!(r0 >= 0.0)) flags |= kFlagNonFinite;
+          double v1, v2, v3;
+          apply_sources(c0, nsrc - 1, g.small_eps);
+          gravity_source0(c0, go1, go2, go3, dth, g.small_eps, v1, v2, v3);
         } else {
-          rate = fmax(rate, r0);
-          if (!(r0 >= 0.0)) flags |= kFlagNonFinite;
+          const SharedDiv q0(c0.d);
+#pragma unroll 1
+          for (int k = 0; k < nsrc; ++k)
+            c0.E = source_energy_q(q0, c0.m1, c0.m2, c0.m3, c0.E, g.small_eps);
         }
-      }
-      const long long o = g.base + gx + (long long)gy * g.sy + (long long)z * g.sz;
+        double n[5];
+        // flux_ang updates the transformed momenta (flux_ang.f90:44-62, 149-246)
+        if (ANG) ang_to(g, gx, gy, c0.m1, c0.m2, c0.m1, c0.m2);
+        if (is0) {
+          n[0] = c0.d + ft[0];
+          n[1] = c0.m1 + ft[1];
+          n[2] = c0.m2 + ft[2];
+          n[3] = c0.m3 + ft[3];
+          n[4] = c0.E + ft[4];
+        } else {
+          if (ANG) ang_to(g, gx, gy, c1.m1, c1.m2, c1.m1, c1.m2);
+          n[0] = kHalf * (c0.d + c1.d + ft[0]);
+          n[1] = kHalf * (c0.m1 + c1.m1 + ft[1]);
+          n[2] = kHalf * (c0.m2 + c1.m2 + ft[2]);
+          n[3] = kHalf * (c0.m3 + c1.m3 + ft[3]);
+          n[4] = kHalf * (c0.E + c1.E + ft[4]);
+        }
+        if (ANG) {
+          // back to (m1, m2) (flux_ang.f90:247-270)
+          double cxp, cyp, crp;
+          cell_xyr(g, gx, gy, cxp, cyp, crp);
+          const double tyy = cyp + g.yoff, trr = sqrt(cxp * cxp + tyy * tyy);
+          const double rmom = n[1], angmom = n[2];
+          n[1] = (rmom * cxp - angmom * tyy / trr) / trr;
+          n[2] = (rmom * tyy + angmom * cxp / trr) / trr;
+        }
+        floors(n[0], n[1], n[2], n[3], n[4], g.small_rho, g.small_eps);
+        if (!(isfinite(n[0]) && isfinite(n[1]) && isfinite(n[2]) && isfinite(n[3]) &&
+              isfinite(n[4])))
+          flags |= kFlagNonFinite;
+        if (!is0) {
+          // state/velocity after flux(1) and after source(1) (main.f90:372-380,490-515);
+          // without a force every division here is by the new density: one
+          // reciprocal and one window check for all of them (epi_fast)
+          double u1, u2, u3, r0 = 0.0;
+          if (GRAV) {
+            const SharedDiv qn(n[0]);
+            u1 = qn(n[1]);
+            u2 = qn(n[2]);
+            u3 = qn(n[3]);
+          } else if (TAB) {
+            epi_tab<POW2>(g, a.eos, n, u1, u2, u3, r0);
+          } else if (!epi_fast<POW2>(g, n, u1, u2, u3, r0)) {
+            epi_ieee<POW2>(g, n, u1, u2, u3, r0);
+          }
+          if (n[0] < kLowRho) flags |= kFlagLowRho;
+          if (fabs(u1) > g.vlimit || fabs(u2) > g.vlimit || fabs(u3) > g.vlimit)
+            flags |= kFlagVlimit;
+          if (GRAV) {
+            // source(1) with the force (main.f90:471): the planes take its result,
+            // the velocity it read goes to UC for state() at the step's end
+            // (main.f90:513-514), and the Courant rate of the next step is taken
+            // with the velocity after it (main.f90:515)
+            a.UC[o] = u1;
+            a.UC[PS + o] = u2;
+            a.UC[2 * PS + o] = u3;
+            source_gravity(n[0], n[1], n[2], n[3], n[4], go1, go2, go3, u1, u2, u3, dth,
+                           g.small_eps);
+            const double w1 = n[1] / n[0], w2 = n[2] / n[0], w3 = n[3] / n[0];
+            if (fabs(w1) > g.vlimit || fabs(w2) > g.vlimit || fabs(w3) > g.vlimit)
+              flags |= kFlagVlimit;
+            if (!(isfinite(n[1]) && isfinite(n[2]) && isfinite(n[3]) && isfinite(n[4])))
+              flags |= kFlagNonFinite;
+            const double pA = eos_pressure(n[0], n[4], w1, w2, w3, g.gm1, g.small_eps);
+            const double r0 = courant_rate<POW2>(n[0], pA, g.gam, w1, w2, w3, g.dx, g.dy, g.dz,
+                                                 g.idx, g.idy, g.idz);
+            rate = at_least(r0, rate);
+            if (!(r0 >= 0.0)) flags |= kFlagNonFinite;
+          } else {
+            rate = at_least(r0, rate);
+            if (!(r0 >= 0.0)) flags |= kFlagNonFinite;
+          }
+        }
 #pragma unroll
-      for (int q = 0; q < 5; ++q) a.out[q * PS + o] = n[q];
-      if (THREED) {
-#pragma unroll
-        for (int q = 0; q < 5; ++q) zs(q) = zs(5 + q);
-        Pk = Pk1;
-        Pk1 = P2;
+        for (int q = 0; q < 5; ++q) a.out[q * PS + o] = n[q];
       }
     }
-    __syncthreads();
   }
 
   // block reductions of the Courant rate and the status bits
+  __syncthreads();
   const unsigned wf = __reduce_or_sync(0xffffffffu, flags);
   const double wr = warp_max(rate);
   if ((tid & 31) == 0) {
@@ -915,12 +918,12 @@ struct ShapeSel<3> {
 // exact for any spacing).  SH: the tile shape (Shape0 or Shape1; Shape2 with the
 // tabulated EOS, Shape3 with angular-momentum fluxing).
 template <int STAGE, int PM, bool THREED, bool GRAV = false, int SH = 0>
-__global__ void __launch_bounds__(NT, 65536 / (NT * 128)) k_stage(StageArgs a) {
+__global__ void __launch_bounds__(kStageThreads, 2) k_stage(StageArgs a) {
   using S = typename ShapeSel<SH>::type;
   extern __shared__ double sm[];
   __shared__ Geom sg;
-  __shared__ double red_rate[NT / 32];
-  __shared__ unsigned red_flags[NT / 32];
+  __shared__ double red_rate[kStageThreads / 32];
+  __shared__ unsigned red_flags[kStageThreads / 32];
   const Tile t = a.tiles[blockIdx.x];
   if (threadIdx.x == 0) sg = a.geom[t.box];
   __syncthreads();
@@ -928,12 +931,7 @@ __global__ void __launch_bounds__(NT, 65536 / (NT * 128)) k_stage(StageArgs a) {
   if (!C->active) return;
   const double dt = C->dt;
   const int nsrc = a.nsrc > 0 ? a.nsrc : C->nsrc;
-  const bool full = (t.x0 + S::TX <= sg.ax1 - sg.ax0) && (t.y0 + S::TY <= sg.ay1 - sg.ay0);
-  constexpr bool P2 = PM == 1;
-  if (full)
-    stage_tile<S, STAGE, P2, THREED, true, GRAV>(a, t, sg, C, dt, nsrc, sm, red_rate, red_flags);
-  else
-    stage_tile<S, STAGE, P2, THREED, false, GRAV>(a, t, sg, C, dt, nsrc, sm, red_rate, red_flags);
+  stage_tile<S, STAGE, PM == 1, THREED, GRAV>(a, t, sg, C, dt, nsrc, sm, red_rate, red_flags);
 }
 
 // A batched box's clock at the start of a step (dt control of main.f90:266-281
@@ -1021,17 +1019,17 @@ __device__ __forceinline__ void persistent_tile(int stage, const StageArgs& a, c
                                                 const Geom& g, Ctrl* C, double dt, int nsrc,
                                                 double* sm, double* red_rate,
                                                 unsigned* red_flags) {
-  stage_tile<S, 2, PM == 1, THREED, false, false, true>(a, t, g, C, dt, nsrc, sm, red_rate,
+  stage_tile<S, 2, PM == 1, THREED, false, true>(a, t, g, C, dt, nsrc, sm, red_rate,
                                                         red_flags, stage);
 }
 
 template <int PM, bool THREED, int SH>
-__global__ void __launch_bounds__(NT, 65536 / (NT * 128)) k_batch_persistent(PersistArgs p) {
+__global__ void __launch_bounds__(kStageThreads, 2) k_batch_persistent(PersistArgs p) {
   using S = typename ShapeSel<SH>::type;
   extern __shared__ double sm[];
   __shared__ Geom sg;
-  __shared__ double red_rate[NT / 32];
-  __shared__ unsigned red_flags[NT / 32];
+  __shared__ double red_rate[kStageThreads / 32];
+  __shared__ unsigned red_flags[kStageThreads / 32];
   __shared__ long long s_item;
   __shared__ int s_run, s_nsrc;
   __shared__ double s_dt;
@@ -1119,11 +1117,11 @@ static cudaError_t launch_persistent_t(const PersistArgs& p, int nbox, cudaStrea
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
     return e;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, NT, smem)) != cudaSuccess)
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kStageThreads, smem)) != cudaSuccess)
     return e;
   const int blocks = std::max(1, per_sm) * sms;
   k_persist_init<<<(nbox + 127) / 128, 128, 0, s>>>(p, nbox);
-  k_batch_persistent<PM, THREED, SH><<<blocks, NT, smem, s>>>(p);
+  k_batch_persistent<PM, THREED, SH><<<blocks, kStageThreads, smem, s>>>(p);
   if (blocks_out) *blocks_out = blocks;
   return cudaGetLastError();
 }
@@ -1179,7 +1177,7 @@ static cudaError_t launch_stage_t(const StageArgs& a, int ntiles, cudaStream_t s
   cudaError_t e = ensure_dyn_smem((const void*)k_stage<STAGE, PM, THREED, GRAV, SH>, smem);
   if (e != cudaSuccess) return e;
   if (ntiles <= 0) return cudaSuccess;
-  k_stage<STAGE, PM, THREED, GRAV, SH><<<ntiles, NT, smem, s>>>(a);
+  k_stage<STAGE, PM, THREED, GRAV, SH><<<ntiles, kStageThreads, smem, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -1593,8 +1591,8 @@ __global__ void k_phase_states(Geom g, PhaseArrays a, Ctrl* ctrl) {
       sl[NQ - 1] = slope3(c[2 * n + im], c[2 * n + i], c[2 * n + ip]);
     }
     const double ud = u[dir * n + i];
-    const double lp = fmax(ud + sound, 0.0) * dt / ds[dir];
-    const double lm = fmin(ud - sound, 0.0) * dt / ds[dir];
+    const double lp = at_least(ud + sound, 0.0) * dt / ds[dir];
+    const double lm = at_most(ud - sound, 0.0) * dt / ds[dir];
     double q[NQ];
     q[0] = d0; q[1] = u[i]; q[2] = u[n + i]; q[3] = u[2 * n + i];
     q[4] = a.p[i]; q[5] = eps0; q[6] = a.adindx[i];
@@ -1676,8 +1674,8 @@ __device__ __forceinline__ void phase_face(const double* S, long long n, int dir
   fr[4] = (sr[4] + pr) * vr;
   const double cr = sqrt(gr * pr / dr);
   const double cl = sqrt(gl * pl / dl);
-  const double ap = fmax(fmax(0.0, vr + cr), vl + cl);
-  const double am = fmax(fmax(0.0, -(vr - cr)), -(vl - cl));
+  const double ap = at_least(vl + cl, at_least(vr + cr, 0.0));
+  const double am = at_least(-(vl - cl), at_least(-(vr - cr), 0.0));
   for (int k = 0; k < 5; ++k) F[k] = (ap * fl[k] + am * fr[k] - ap * am * (sr[k] - sl[k])) / (ap + am);
 }
 
@@ -2184,7 +2182,7 @@ int stage_blocks_per_sm(int stage, int pm, bool threed, int shape) {
                    : (threed ? (const void*)k_stage<1, 0, true> : (const void*)k_stage<1, 0, false>);
   }
   if (ensure_dyn_smem(fn, smem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, NT, smem) != cudaSuccess) {
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kStageThreads, smem) != cudaSuccess) {
     cudaGetLastError();
     return 1;
   }
