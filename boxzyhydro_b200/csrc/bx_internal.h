@@ -106,9 +106,7 @@ struct TileShape {
   // (5 + 5) and the plus z-state carried to the next plane (NSF), kept in
   // shared memory so the x/y phases have the registers
   static constexpr int NZS = 10 + NSF;
-  // one 16-bit table entry per state item (stage_tile)
-  static constexpr int SMEM_DOUBLES = NPF * NP + 2 * NSF * (NSX + NSY) + NZS * NOWN +
-                                      (NSX + NSY + 3) / 4;
+  static constexpr int SMEM_DOUBLES = NPF * NP + 2 * NSF * (NSX + NSY) + NZS * NOWN;
   static_assert(TX * TY <= NT && NT % 32 == 0, "tile larger than the block");
   static_assert(4 * (TX + TY) <= NT, "one halo cell per thread and plane at most");
 };

@@ -343,8 +343,10 @@ __device__ __forceinline__ void ang_to(const Geom& g, int ix, int iy, double m1,
   am = x * m2 - y * m1;
 }
 
-template <bool POW2, bool TAB = false, bool ANG = false>
-__device__ __forceinline__ void dir_states(const Prim& m, const Prim& c, const Prim& p, double ud,
+// the face states of cell c between m and p along an axis: the normal velocity is
+// u1 (the x/y phases, which exchange the velocities for y) or u3 (AX 2)
+template <bool POW2, bool TAB = false, bool ANG = false, int AX = 0>
+__device__ __forceinline__ void dir_states(const Prim& m, const Prim& c, const Prim& p, bool ghost,
                                            double dt, double ds, double ids, FaceState& mi,
                                            FaceState& pl) {
   const double sd = slope3(m.d, c.d, p.d);
@@ -358,7 +360,8 @@ __device__ __forceinline__ void dir_states(const Prim& m, const Prim& c, const P
   // flux_ang's transformed momenta (flux_ang.f90:301-345)
   const double srm = ANG ? slope3(m.rm, c.rm, p.rm) : 0.0;
   const double sam = ANG ? slope3(m.am, c.am, p.am) : 0.0;
-  muscl_states<POW2, TAB, ANG>(c, ud, sd, s1, s2, s3, sp, se, dt, ds, ids, mi, pl, sg, srm, sam);
+  muscl_states<POW2, TAB, ANG>(c, AX == 2 ? c.u3 : c.u1, sd, s1, s2, s3, sp, se, dt, ds, ids, mi,
+                               pl, sg, srm, sam, ghost);
 }
 
 template <int NP, int NPF = 7>
@@ -510,26 +513,30 @@ __device__ __forceinline__ void epi_tab(const Geom& g, const EosDev& eos, const 
 //     and the own cell's update.
 // B and C run both axes through one code, with the velocities along and across
 // the axis in each other's place for y (the HLL flux is the same arithmetic with
-// them exchanged); what an item of a thread reads is worked out once per tile and
-// kept in a table (s_item), not per plane.  A plane takes three barriers: the
+// them exchanged), in three rounds of the block: every thread's own cell along x,
+// along y, and the tile's rim (80 states and 40 faces of 32 x 8 columns).  What a
+// round reads is worked out once per tile.  A plane takes three barriers: the
 // fluxes go where the states they came from were, so nothing of D is overwritten
 // by A of the next plane.
 //
-// What bounds it (ncu, 128^3, stage 0 / 1): not memory (DRAM 8-12 % busy) but the
-// latency of the FP64 chains at 16 warps per SM, the registers' limit: 53 / 52 %
-// of issue slots, 45 % of the FP64 pipe; of 7.1 warp cycles per instruction 1.65
-// wait on a fixed latency, 1.2 at a barrier, 0.5 for the FP64 pipe, 0.6-0.8 for
-// global loads.  So the gains lie in fewer instructions and no spills.  Measured
-// per 256^3 step on one box: 4.68 ms with a code path per axis, every bound by
-// fmax and fluxes over the primitives (a fourth barrier); 4.64 with both axes in
-// one path and compare-and-select bounds (2420 and 2690 executed instructions per
-// cell); 4.20 with the item table, the places of own and halo cells worked out
-// once per tile (2240 and 2400) and the fluxes' dividing code once; 4.11 with three
-// barriers.  The halo cell's loads are issued after the own cell's arithmetic:
-// both at once spill 84-124 bytes per thread and measured 4.57 ms.  A rim warp
-// that takes all halo work, with states and fluxes passed by shuffles, measured
-// 5.7 ms (its chain of five primitives paces the block, and 140-190 KB of code
-// against 60 miss in the instruction cache).
+// What bounds it (ncu, 128^3): not memory (DRAM 8-12 % busy) but the latency of
+// the FP64 chains at 16 warps per SM, the registers' limit: 53 % of issue slots
+// and 45 % of the FP64 pipe; of 7.1 warp cycles per instruction 1.65 wait on a
+// fixed latency, 1.2 at a barrier, 0.5 for the FP64 pipe, 0.6-0.8 for global
+// loads.  So the gains lie in fewer instructions and no spills.  Measured per
+// 256^3 step on one box: 4.68 ms with a code path per axis, every bound by fmax
+// and fluxes over the primitives (a fourth barrier); 4.64 with both axes in one
+// path and compare-and-select bounds (2420 and 2690 executed instructions per
+// cell in stage 0 and 1); 4.20 with the places of own and halo cells worked out
+// once per tile and a table of the items (2240 and 2400); 4.11 with three
+// barriers; 3.96 with the items as rounds and no branch for ghosts' states (2120
+// and 2300); 3.80 with stage 1's prefetch of the step input moved out of phase A,
+// which took its last spills; 3.78 with the rim
+// going to threads without a column first.  The halo cell's loads are issued after the own
+// cell's arithmetic: both at once spill 84-124 bytes per thread and measured 4.57
+// against 4.20 ms.  A rim warp that takes all halo work, with states and fluxes
+// passed by shuffles, measured 5.7 ms (its chain of five primitives paces the
+// block, and 140-190 KB of code against 60 miss in the instruction cache).
 // dt: the step's full dt; nsrc: the sources the stage input is short of (both
 // read from the box's control block by the caller).  CG: inputs through L2 (the
 // persistent batched kernel).
@@ -543,14 +550,13 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
   constexpr int TX = S::TX, TY = S::TY, NT = S::NT, PW = S::PW, NP = S::NP;
   constexpr bool TAB = S::TAB, ANG = S::ANG;
   constexpr int NPF = S::NPF, NSF = S::NSF, NFQ = S::NFQ, NOWN = S::NOWN;
-  constexpr int NSX = S::NSX, NS = S::NSX + S::NSY, NFX = S::NFX, NF = S::NFX + S::NFY;
+  constexpr int NSX = S::NSX, NS = S::NSX + S::NSY;
   double* SP = sm;                  // [NPF][TY+4][TX+4] primitives of the plane
   double* SS = sm + NPF * NP;       // [2 NSF] minus, then plus: x [TY][TX+2], y [TY+2][TX]
   // face fluxes: each state is read by one face only, so a face's flux takes the
   // place of the plus state below it
   double* FF = SS + NSF * NS;
   double* ZS = SS + 2 * NSF * NS;   // [10 + NSF][NOWN]: z flux, its difference over the plane, plus z state
-  unsigned short* s_item = reinterpret_cast<unsigned short*>(ZS + (10 + NSF) * NOWN);  // [NS]
   const double dth = dt * kHalf;  // the sources' half step (main.f90:282,471)
 
   const int tid = threadIdx.x;
@@ -565,20 +571,33 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
   unsigned flags = 0;
   double rate = 0.0;
 
-  // the table of state items: the cell in SP
-  for (int i = tid; i < NS; i += NT) {
-    const int ax = i >= NSX, k = i - NSX;
-    const int cy = ax ? k / TX - 1 : i / (TX + 2), cx = ax ? k % TX : i % (TX + 2) - 1;
-    const int f = ax ? by0 + cy : bx0 + cx;
-    const bool ghost = f < (ax ? g.ay0 : g.ax0) || f >= (ax ? g.ay1 : g.ax1);
-    s_item[i] = (unsigned short)(((cy + 2) * PW + cx + 2) | (ax ? kItemY : 0u) |
-                                 (ghost ? kItemGhost : 0u) |
-                                 (cx < w + 1 - ax && cy < h + ax ? kItemIn : 0u));
+  // the items of this thread in B and C: its own cell's states and lower faces,
+  // x then y, and the tile's rim, which the threads without a column take first
+  const int sc = (ty + 2) * PW + tx + 2;                        // the own cell in SP
+  const int lx = ty * (TX + 2) + tx, ly = NSX + ty * TX + tx;  // the states below its faces
+  const int rt = (tid + NT - NOWN) % NT;
+  unsigned rim_b = 0, rim_c = 0;  // state: cell in SP, flags, place in SS << 16; face: low state
+  if (rt < 2 * TX) {
+    const int cx = rt % TX, cy = rt < TX ? h : -1, f = by0 + cy;
+    if (cx < w) {
+      rim_b = (unsigned)((cy + 2) * PW + cx + 2) | kItemIn | kItemY |
+              (f < g.ay0 || f >= g.ay1 ? kItemGhost : 0u) |
+              (unsigned)(NSX + (cy + 1) * TX + cx) << 16;
+      if (rt < TX) rim_c = (unsigned)(NSX + h * TX + cx) | kItemIn | kItemY;
+    }
+  } else if (rt < 2 * TX + 2 * TY) {
+    const int k = rt - 2 * TX, cy = k >> 1, cx = (k & 1) ? w : -1, f = bx0 + cx;
+    if (cy < h) {
+      rim_b = (unsigned)((cy + 2) * PW + cx + 2) | kItemIn |
+              (f < g.ax0 || f >= g.ax1 ? kItemGhost : 0u) |
+              (unsigned)(cy * (TX + 2) + cx + 1) << 16;
+      if (k & 1) rim_c = (unsigned)(cy * (TX + 2) + w) | kItemIn;
+    }
   }
 
   // the halo cell of this thread (those without a column first), if any
   static_assert(4 * (TX + TY) <= NT, "one halo cell per thread and plane at most");
-  Place hp{0, false, false, false};
+  long long hpc = 0;
   int hc = -1;  // its place in SP
   {
     const int i = (tid + NT - NOWN) % NT;
@@ -596,9 +615,10 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
       in = j < 4 && cx < w;
     }
     if (in) {
-      hp = place_of(g, bx0 + cx, by0 + cy, g.az0);
-      hp.c -= (long long)g.az0 * g.sz;
-      hc = (cy + 2) * PW + cx + 2;
+      const Place p = place_of(g, bx0 + cx, by0 + cy, g.az0);
+      hpc = p.c - (long long)g.az0 * g.sz;
+      // (a halo cell of the x/y halo is beyond one wall at most)
+      hc = ((cy + 2) * PW + cx + 2) | (p.fx ? 1 << 12 : 0) | (p.fy ? 1 << 13 : 0);
     }
   }
   const long long co = g.base + gx + (long long)gy * g.sy;  // the own column
@@ -639,10 +659,6 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
       if (own) {
         // towards L2: the step input that stage 1's update reads at the end of
         // this plane, and the own column's loads of the next plane
-        if (!is0 && plane) {
-#pragma unroll
-          for (int q = 0; q < 5; ++q) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.X + o + q * PS));
-        }
         if (THREED && z + 3 < g.az1) {
           const long long o3 = o + 3 * g.sz;
           const double* B = is0 ? a.X : a.Y;
@@ -656,7 +672,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
         if (THREED) P2 = prim_at(ro, gx, gy);
         else Pk = prim_at(ro, gx, gy);
         if (plane) {
-          put_prim<NP, NPF>(SP, (ty + 2) * PW + tx + 2, Pk);
+          put_prim<NP, NPF>(SP, sc, Pk);
           // the guards look at every interior cell where it is an own cell
           if (Pk.d < kLowRho) flags |= kFlagLowRho;
           if (fabs(Pk.u1) > g.vlimit || fabs(Pk.u2) > g.vlimit || fabs(Pk.u3) > g.vlimit)
@@ -670,21 +686,17 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
         }
       }
       if (halo) {
-        Place p = hp;
-        p.c += (long long)z * g.sz;
+        const Place p{hpc + (long long)z * g.sz, (hc & (1 << 12)) != 0, (hc & (1 << 13)) != 0, false};
         rh = load_raw<STAGE, GRAV, CG>(a, p, rs);
 
-        const int cy = hc / PW - 2, cx = hc % PW - 2;
-        put_prim<NP, NPF>(SP, hc, prim_at(rh, bx0 + cx, by0 + cy));
+        const int k = hc & 0xfff, cy = k / PW - 2, cx = k % PW - 2;
+        put_prim<NP, NPF>(SP, k, prim_at(rh, bx0 + cx, by0 + cy));
       }
       // the z states of the cell above and the z face between
       if (THREED && own) {
         FaceState mz, pz;
-        if (z + 1 < g.az0 || z + 1 >= g.az1) {
-          ghost_states(Pk1, mz, pz);
-        } else {
-          dir_states<POW2, TAB, ANG>(Pk, Pk1, P2, Pk1.u3, dt, g.dz, g.idz, mz, pz);
-        }
+        dir_states<POW2, TAB, ANG, 2>(Pk, Pk1, P2, z + 1 < g.az0 || z + 1 >= g.az1, dt, g.dz,
+                                      g.idz, mz, pz);
         Pk = Pk1;
         Pk1 = P2;
         if (z >= z0 - 1) {
@@ -709,35 +721,42 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
     if (plane) {
       __syncthreads();
       // ---- B: x and y face states of the plane
-      for (int i = tid; i < NS; i += NT) {
-        const unsigned e = s_item[i];
-        if (!(e & kItemIn)) continue;
-        const int ax = (e & kItemY) ? 1 : 0, c = e & 0xfffu, st = ax ? PW : 1;
-        const Prim q = get_prim_along<NP, NPF>(SP, c, ax);
-        FaceState mi, pl;
-        if (e & kItemGhost) {
-          ghost_states(q, mi, pl);
-        } else {
-          dir_states<POW2, TAB, ANG>(get_prim_along<NP, NPF>(SP, c - st, ax), q,
-                                     get_prim_along<NP, NPF>(SP, c + st, ax), q.u1, dt,
-                                     ax ? g.dy : g.dx, ax ? g.idy : g.idx, mi, pl);
+      {
+        unsigned e = own ? (unsigned)sc | kItemIn : rim_b;
+        int k = own ? lx + 1 : (int)(rim_b >> 16);
+#pragma unroll 1
+        for (int it = 0; it < 3; ++it) {
+          if (e & kItemIn) {
+            const int ax = (e & kItemY) ? 1 : 0, c = e & 0xfffu, st = ax ? PW : 1;
+            FaceState mi, pl;
+            dir_states<POW2, TAB, ANG>(
+                get_prim_along<NP, NPF>(SP, c - st, ax), get_prim_along<NP, NPF>(SP, c, ax),
+                get_prim_along<NP, NPF>(SP, c + st, ax), (e & kItemGhost) != 0, dt,
+                ax ? g.dy : g.dx, ax ? g.idy : g.idx, mi, pl);
+            put_fs<NSF>(SS, NS, k, mi);
+            put_fs<NSF>(FF, NS, k, pl);
+          }
+          if (!own) break;
+          e = it ? rim_b : e | kItemY;
+          k = it ? (int)(rim_b >> 16) : ly + TX;
         }
-        put_fs<NSF>(SS, NS, i, mi);
-        put_fs<NSF>(FF, NS, i, pl);
       }
       __syncthreads();
       // ---- C: x and y face fluxes (face f lies between cells f-1 and f)
-      for (int i = tid; i < NF; i += NT) {
-        const int ax = i >= NFX, k = i - NFX;
-        const int cy = ax ? k / TX : i / (TX + 1), cx = ax ? k % TX : i % (TX + 1);
-        if (cx >= w + 1 - ax || cy >= h + ax) continue;
-        const int lo = ax ? NSX + k : i + cy;
+      unsigned ec = own ? (unsigned)lx | kItemIn : rim_c;
+#pragma unroll 1
+      for (int it = 0; it < 3; ++it) {
+        const unsigned e = ec;
+        ec = !own ? 0u : it ? rim_c : (unsigned)ly | kItemIn | kItemY;
+        if (!(e & kItemIn)) continue;
+        const int ax = (e & kItemY) ? 1 : 0, lo = e & 0xfffu;
         // the plus state of the cell below the face and the minus state of the one above
         const FaceState L = get_fs<NSF>(FF, NS, lo);
         const FaceState R = get_fs<NSF>(SS, NS, lo + (ax ? TX : 1));
         double F[NFQ];
         if constexpr (ANG) {
           // the momentum fluxes for both cells of the face (their own centres)
+          const int cy = ax ? (lo - NSX) / TX : lo / (TX + 2), cx = lo - (ax ? NSX + cy * TX : cy * (TX + 2));
           double xl, yl, rl, xh, yh, rh;
           cell_xyr(g, bx0 + cx - 1 + ax, by0 + cy - ax, xl, yl, rl);
           cell_xyr(g, bx0 + cx, by0 + cy, xh, yh, rh);
@@ -762,6 +781,12 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
       __syncthreads();
     }
 
+    if (!is0 && own && z + 1 < z1 && (!THREED || z + 1 >= z0)) {
+      // towards L2: the step input that stage 1's update reads on the next plane
+      const double* xn = a.X + o + g.sz;
+#pragma unroll
+      for (int q = 0; q < 5; ++q) asm volatile("prefetch.global.L2 [%0];" ::"l"(xn + q * PS));
+    }
     // ---- D: the z face above the own cell, and its update (flux.f90:186-230)
     if (own) {
       Cons c0, c1;
@@ -779,9 +804,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
           // with flux_ang the momentum fluxes of this cell's plus faces are the
           // versions for their low cell (planes 5, 6)
           const int qp = (ANG && (q == 1 || q == 2)) ? q + 4 : q;
-          const int fx = ty * (TX + 2) + tx, fy = NSX + ty * TX + tx;
-          const double dfx = FF[qp * NS + fx + 1] - FF[q * NS + fx];
-          const double dfy = FF[qp * NS + fy + TX] - FF[q * NS + fy];
+          const double dfx = FF[qp * NS + lx + 1] - FF[q * NS + lx];
+          const double dfy = FF[qp * NS + ly + TX] - FF[q * NS + ly];
           double sum = g.ayz * dfx + g.axz * dfy;
           if (THREED) sum = sum + g.axy * zs(5 + q);
           ft[q] = POW2 ? -sum * dt * g.ivol : cdiv(-sum * dt, g.vol, g.ivol);
