@@ -82,11 +82,10 @@ struct Tile {
 // path's; the batched path's autotuner may pick shape 1.  32 x 8 columns in 256
 // threads, two blocks per SM: 16 x 14 in 256 measured 5 % slower, 32 x 16 in 512
 // (one block per SM, its barriers without a second block to hide them) 2 %.
-constexpr int kStageThreads = 256;
-template <int TX_, int TY_, int MODE_ = 0>
+template <int TX_, int TY_, int MODE_ = 0, int NT_ = 256>
 struct TileShape {
   static constexpr int TX = TX_, TY = TY_;
-  static constexpr int NT = kStageThreads;
+  static constexpr int NT = NT_;
   // MODE 1 (TAB): the tabulated EOS, whose gamma is a reconstructed primitive;
   // MODE 2 (ANG): angular-momentum fluxing, whose radial and angular momenta
   // are reconstructed primitives and whose x/y face fluxes of the two momentum
@@ -100,11 +99,9 @@ struct TileShape {
   static constexpr int NP = (TY + 4) * PW;   // prim plane cells
   static constexpr int NSX = TY * (TX + 2);  // x-state cells
   static constexpr int NSY = (TY + 2) * TX;  // y-state cells
-  static constexpr int NFX = TY * (TX + 1);  // x faces
-  static constexpr int NFY = (TY + 1) * TX;  // y faces
-  // per-column z-pipeline slots (3-D): the z flux below and above the own cell
-  // (5 + 5) and the plus z-state carried to the next plane (NSF), kept in
-  // shared memory so the x/y phases have the registers
+    // per-column z-pipeline slots (3-D): the z flux below the own cell and its
+  // difference over the cell (5 + 5) and the plus z-state carried to the next
+  // plane (NSF), kept in shared memory so the x/y phases have the registers
   static constexpr int NZS = 10 + NSF;
   static constexpr int SMEM_DOUBLES = NPF * NP + 2 * NSF * (NSX + NSY) + NZS * NOWN;
   static_assert(TX * TY <= NT && NT % 32 == 0, "tile larger than the block");
@@ -113,10 +110,13 @@ struct TileShape {
 using Shape0 = TileShape<32, 8>;
 using Shape1 = TileShape<16, 16>;
 // the tabulated EOS and angular-momentum fluxing (single grids only): 32 x 6
-// columns, so the larger primitive and face-state sets still fit two blocks
-// per SM
-using Shape2 = TileShape<32, 6, 1>;
-using Shape3 = TileShape<32, 6, 2>;
+// columns, so the larger primitive and face-state sets still fit two blocks per
+// SM, and a thread per column: with 192 threads a thread may hold 168 registers and
+// nothing spills (with 256 threads, 128 registers: 172 bytes per thread with
+// flux_ang, 76 with the tables; measured 569 against 501 us and 629 against 611
+// per 96^3 step; 224 threads get the same 128 registers)
+using Shape2 = TileShape<32, 6, 1, 192>;
+using Shape3 = TileShape<32, 6, 2, 192>;
 constexpr int kNumShapes = 2;  // the shapes the batched autotuner chooses among
 // the x and y extents of tile shape `shape`
 inline int shape_tx(int shape) {
@@ -124,6 +124,10 @@ inline int shape_tx(int shape) {
 }
 inline int shape_ty(int shape) {
   return shape == 3 ? Shape3::TY : shape == 2 ? Shape2::TY : shape == 1 ? Shape1::TY : Shape0::TY;
+}
+
+inline int shape_threads(int shape) {
+  return shape == 3 ? Shape3::NT : shape == 2 ? Shape2::NT : shape == 1 ? Shape1::NT : Shape0::NT;
 }
 
 // ghost-fill tables: per ghost (index order), destination cell, source cell and

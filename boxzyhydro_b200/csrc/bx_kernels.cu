@@ -942,12 +942,12 @@ struct ShapeSel<3> {
 // exact for any spacing).  SH: the tile shape (Shape0 or Shape1; Shape2 with the
 // tabulated EOS, Shape3 with angular-momentum fluxing).
 template <int STAGE, int PM, bool THREED, bool GRAV = false, int SH = 0>
-__global__ void __launch_bounds__(kStageThreads, 2) k_stage(StageArgs a) {
+__global__ void __launch_bounds__(ShapeSel<SH>::type::NT, 2) k_stage(StageArgs a) {
   using S = typename ShapeSel<SH>::type;
   extern __shared__ double sm[];
   __shared__ Geom sg;
-  __shared__ double red_rate[kStageThreads / 32];
-  __shared__ unsigned red_flags[kStageThreads / 32];
+  __shared__ double red_rate[ShapeSel<SH>::type::NT / 32];
+  __shared__ unsigned red_flags[ShapeSel<SH>::type::NT / 32];
   const Tile t = a.tiles[blockIdx.x];
   if (threadIdx.x == 0) sg = a.geom[t.box];
   __syncthreads();
@@ -1048,12 +1048,12 @@ __device__ __forceinline__ void persistent_tile(int stage, const StageArgs& a, c
 }
 
 template <int PM, bool THREED, int SH>
-__global__ void __launch_bounds__(kStageThreads, 2) k_batch_persistent(PersistArgs p) {
+__global__ void __launch_bounds__(ShapeSel<SH>::type::NT, 2) k_batch_persistent(PersistArgs p) {
   using S = typename ShapeSel<SH>::type;
   extern __shared__ double sm[];
   __shared__ Geom sg;
-  __shared__ double red_rate[kStageThreads / 32];
-  __shared__ unsigned red_flags[kStageThreads / 32];
+  __shared__ double red_rate[ShapeSel<SH>::type::NT / 32];
+  __shared__ unsigned red_flags[ShapeSel<SH>::type::NT / 32];
   __shared__ long long s_item;
   __shared__ int s_run, s_nsrc;
   __shared__ double s_dt;
@@ -1141,11 +1141,11 @@ static cudaError_t launch_persistent_t(const PersistArgs& p, int nbox, cudaStrea
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
     return e;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kStageThreads, smem)) != cudaSuccess)
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, ShapeSel<SH>::type::NT, smem)) != cudaSuccess)
     return e;
   const int blocks = std::max(1, per_sm) * sms;
   k_persist_init<<<(nbox + 127) / 128, 128, 0, s>>>(p, nbox);
-  k_batch_persistent<PM, THREED, SH><<<blocks, kStageThreads, smem, s>>>(p);
+  k_batch_persistent<PM, THREED, SH><<<blocks, ShapeSel<SH>::type::NT, smem, s>>>(p);
   if (blocks_out) *blocks_out = blocks;
   return cudaGetLastError();
 }
@@ -1201,7 +1201,7 @@ static cudaError_t launch_stage_t(const StageArgs& a, int ntiles, cudaStream_t s
   cudaError_t e = ensure_dyn_smem((const void*)k_stage<STAGE, PM, THREED, GRAV, SH>, smem);
   if (e != cudaSuccess) return e;
   if (ntiles <= 0) return cudaSuccess;
-  k_stage<STAGE, PM, THREED, GRAV, SH><<<ntiles, kStageThreads, smem, s>>>(a);
+  k_stage<STAGE, PM, THREED, GRAV, SH><<<ntiles, ShapeSel<SH>::type::NT, smem, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -2206,7 +2206,7 @@ int stage_blocks_per_sm(int stage, int pm, bool threed, int shape) {
                    : (threed ? (const void*)k_stage<1, 0, true> : (const void*)k_stage<1, 0, false>);
   }
   if (ensure_dyn_smem(fn, smem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kStageThreads, smem) != cudaSuccess) {
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, shape_threads(shape), smem) != cudaSuccess) {
     cudaGetLastError();
     return 1;
   }
