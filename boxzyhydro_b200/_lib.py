@@ -106,6 +106,8 @@ def lib():
                                                C.POINTER(C.c_ulonglong), dp, dp]),
         "bx_check_root": (C.c_int, [vp, C.c_ulonglong, C.c_ulonglong, C.c_ulonglong, C.c_int,
                                     C.POINTER(C.c_ulonglong), dp]),
+        "bx_check_log_steps": (C.c_int, [C.c_ulonglong, C.c_ulonglong, C.c_double, C.c_double,
+                                         C.c_int, C.POINTER(C.c_ulonglong), dp]),
         "bx_ghost_fill_noalloc": (C.c_int, [vp, C.c_int64, vp, vp, vp, C.c_int64, vp]),
         "bx_noalloc_last_error": (C.c_char_p, []),
         "bx_batch_create": (C.c_int, [C.c_int32, C.POINTER(BxParams), C.POINTER(H)]),

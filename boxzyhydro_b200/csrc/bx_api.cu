@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <string>
 
 #include "bx_internal.h"
@@ -574,15 +575,38 @@ int bx_set_eos_table(bx_handle* h, const bx_eos_table* t) {
   if (!h->g.tab) return set_err(h, BX_ERR_STATE, "the grid was created with H2STAT = -1");
   if (int r = to_phase(h)) return r;
   const long long n2 = (long long)t->neos * t->neos_rho, nr = t->neos_rho;
+  std::vector<double> host;
+  try {
+    host.assign((size_t)(8 * (n2 + nr)), 0.0);
+  } catch (const std::exception&) {
+    return set_err(h, BX_ERR_NOMEM, "no host memory for the EOS tables");
+  }
+  for (long long r = 0; r < nr; ++r) {
+    const long long r0 = r * t->neos;
+    for (long long k = 0; k < t->neos; ++k) {
+      double* p = host.data() + 8 * (r0 + k);
+      const double* T[3] = {t->gamma_table2 + r0, t->muc_table2 + r0, t->tk_table2 + r0};
+      const double* E = t->eng_table2 + r0;
+      p[0] = E[k];
+      for (int q = 0; q < 3; ++q) {
+        p[1 + 2 * q] = T[q][k];
+        if (k + 1 < t->neos) p[2 + 2 * q] = (T[q][k + 1] - T[q][k]) / (E[k + 1] - E[k]);
+      }
+    }
+    double* p = host.data() + 8 * (n2 + r);
+    const long long rp = std::min(r + 1, nr - 1);
+    const bool other = !(t->rho_table[r] == t->rho_table[rp]);
+    p[1] = t->deng_eos_array[r];
+    p[2] = t->eng_table2[r0];
+    p[3] = t->eng_table2[r0 + t->neos - 1];
+    p[4] = t->rho_table[r];
+    p[5] = other ? 1.0 / (t->rho_table[rp] - t->rho_table[r]) : 0.0;
+    p[6] = other ? 1.0 : 0.0;
+  }
   cudaFree(h->d_eos);
   h->d_eos = nullptr;
-  CK(dalloc((void**)&h->d_eos, (4 * n2 + 3 * nr) * sizeof(double)));
-  const double* src[4] = {t->eng_table2, t->gamma_table2, t->muc_table2, t->tk_table2};
-  for (int k = 0; k < 4; ++k)
-    CK(cudaMemcpy(h->d_eos + k * n2, src[k], n2 * sizeof(double), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(h->d_eos + 4 * n2, t->rho_table, nr * sizeof(double), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(h->d_eos + 4 * n2 + nr, t->deng_eos_array, nr * sizeof(double),
-                cudaMemcpyHostToDevice));
+  CK(dalloc((void**)&h->d_eos, host.size() * sizeof(double)));
+  CK(cudaMemcpy(h->d_eos, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice));
   if (!h->pa.muc) {
     CK(dalloc((void**)&h->pa.muc, h->g.ng * sizeof(double)));
     CK(cudaMemset(h->pa.muc, 0, h->g.ng * sizeof(double)));
@@ -594,14 +618,9 @@ int bx_set_eos_table(bx_handle* h, const bx_eos_table* t) {
   e.drho = t->drho_eos;
   e.density_unit = t->density_unit;
   e.tk_bgrnd = t->tk_bgrnd;
-  e.eng2 = h->d_eos;
-  e.gam2 = h->d_eos + n2;
-  e.muc2 = h->d_eos + 2 * n2;
-  e.tk2 = h->d_eos + 3 * n2;
-  e.rho = h->d_eos + 4 * n2;
-  e.deng = h->d_eos + 4 * n2 + nr;
-  e.log_eng1 = h->d_eos + 4 * n2 + 2 * nr;
-  CK(eos_log_rows(e.eng2, e.neos, (int)nr, h->d_eos + 4 * n2 + 2 * nr, h->stream));
+  e.pack = h->d_eos;
+  e.rows = h->d_eos + 8 * n2;
+  CK(eos_log_rows(h->d_eos + 8 * n2, (int)nr, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   // the fused kernels read the tables from here on (not while a force is set)
   update_eligible(h);

@@ -112,6 +112,45 @@ extern "C" int bx_check_root(const double* q, unsigned long long n, unsigned lon
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
+namespace {
+__global__ void k_logcheck(unsigned long long n, unsigned long long seed, double low, double step,
+                           int steps, unsigned long long* bad, double* example) {
+  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
+  for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
+       i += stride) {
+    const unsigned long long z = mix(seed ^ i);
+    // a step's edge (down to two below the table), off by 2^-1 .. 2^-53 of itself or not at all
+    const double edge = exp10(low + ((double)(z % (unsigned)(steps + 3)) - 2.0) * step);
+    const double off = (z >> 40 & 63) > 53 ? 0.0 : ldexp((z >> 39 & 1) ? 1.0 : -1.0, -(int)(z >> 40 & 63));
+    const double x = edge + edge * off;
+    if (bx::log_steps(x, low, step) != (int)((log10(x) - low) / step))
+      if (atomicAdd(bad, 1ull) == 0) example[0] = x;
+  }
+}
+}  // namespace
+
+extern "C" int bx_check_log_steps(unsigned long long n, unsigned long long seed, double low,
+                                  double step, int steps, unsigned long long* mismatches,
+                                  double* example) {
+  if (steps < 1 || !(step > 0.0)) return 1;
+  unsigned long long* bad = nullptr;
+  double* ex = nullptr;
+  if (cudaMalloc(&bad, sizeof(*bad)) != cudaSuccess) return 5;
+  if (cudaMalloc(&ex, sizeof(double)) != cudaSuccess) { cudaFree(bad); return 5; }
+  cudaMemset(bad, 0, sizeof(*bad));
+  cudaMemset(ex, 0, sizeof(double));
+  k_logcheck<<<1184, 256>>>(n, seed, low, step, steps, bad, ex);
+  unsigned long long h = 0;
+  double hx = 0.0;
+  cudaMemcpy(&h, bad, sizeof(h), cudaMemcpyDeviceToHost);
+  cudaMemcpy(&hx, ex, sizeof(hx), cudaMemcpyDeviceToHost);
+  cudaFree(bad);
+  cudaFree(ex);
+  if (mismatches) *mismatches = h;
+  if (example) *example = hx;
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
 extern "C" int bx_check_shared_division(unsigned long long n, unsigned long long seed,
                                          int exp_range, unsigned long long* mismatches,
                                          double* example_a, double* example_d) {

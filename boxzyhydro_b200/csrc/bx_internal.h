@@ -146,18 +146,20 @@ void build_ghost_tables(const bx_params& P, GhostTable& T);
 void fill_geom(const bx_params& P, Geom& g);
 bool is_pow2(double x);
 
-// tabulated EOS on the device (H2STAT >= 0): tables of the eos module
+// tabulated EOS on the device (H2STAT >= 0): the tables of the eos module, an
+// entry's values side by side (64 bytes), and one record per density row
 struct EosDev {
   int neos, neos_rho;
   double log_rho_low, drho, density_unit, tk_bgrnd;
-  const double *eng2, *gam2, *muc2, *tk2;  // (neos, neos_rho), neos fastest
-  const double *rho, *deng;                // (neos_rho)
-  const double* log_eng1;                  // (neos_rho): log10 of each row's first energy
+  // [neos_rho][neos][8]: eng, gamma, dgamma, mu, dmu, T, dT, 0, where dX is
+  // (X(next) - X) / (eng(next) - eng) (0 for a row's last entry)
+  const double* pack;
+  // [neos_rho][8]: log10 of the first energy, deng, the first and the last energy,
+  // rho, 1 / (rho(next) - rho), whether the next row has another density, 0
+  const double* rows;
 };
-// log10 of the first energy of each density row (the value get_gamma2 needs,
-// computed once with the same device function)
-cudaError_t eos_log_rows(const double* eng2, long long neos, int nr, double* out,
-                         cudaStream_t s);
+// fills in the first value of each row record, from its third
+cudaError_t eos_log_rows(double* rows, int nr, cudaStream_t s);
 
 // ---- kernels (bx_kernels.cu)
 struct StageArgs {

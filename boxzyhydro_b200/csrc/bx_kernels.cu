@@ -49,50 +49,53 @@ namespace {
 
 // get_gamma2 (eos.f90:653-699): gamma, mu and T from the tables by the specific
 // internal energy eng = eps/rho, linear in eng within the density row irho, then
-// linear in rho towards row irho+1.  eps is clamped like the reference's.
-__device__ void get_gamma2(const EosDev& e, double& eps, double rho, double& tk, double& m,
-                           double& gam) {
-  int irho = min((int)((log10(rho * e.density_unit) - e.log_rho_low) / e.drho) + 1, e.neos_rho);
+// linear in rho towards row irho+1.  eps is clamped like the reference's.  The
+// quotients of neighbouring entries depend on the tables alone and are formed
+// with them (bx_set_eos_table, the same IEEE divisions), an entry's seven values
+// side by side: 16-byte loads of one or two sectors instead of eight scattered
+// ones, and of the two logarithms and nine divisions a look-up took, one division
+// is left.  Measured per 96^3 step (4.8 look-ups per cell): 611 -> 466 us.
+__device__ __forceinline__ void get_gamma2(const EosDev& e, double& eps, double rho, double& tk,
+                                           double& m, double& gam) {
+  int irho = min(log_steps(rho * e.density_unit, e.log_rho_low, e.drho) + 1, e.neos_rho);
   if (irho < 1) irho = 1;
-  int irhop = irho + 1;
-  if (irhop > e.neos_rho) irhop = irho;
-  const long long ne = e.neos;
-  auto at = [&](const double* t, int ie, int ir) { return t[(ie - 1) + (ir - 1) * ne]; };
-  double eng = eps / rho;
-  // log10 of the row's first energy: precomputed with the same device log10
-  int ientry = (int)((log10(eng) - e.log_eng1[irho - 1]) / e.deng[irho - 1]) + 1;
+  const double2* row = reinterpret_cast<const double2*>(e.rows + 8 * (irho - 1));
+  const double2 r0 = __ldg(row), r1 = __ldg(row + 1), r2 = __ldg(row + 2);  // EosDev::rows
+  const double log_eng1 = r0.x, deng = r0.y, eng1 = r1.x, engn = r1.y;
+  double eng = SharedDiv(rho)(eps);
+  int ientry = log_steps(eng, log_eng1, deng) + 1;
   if (ientry > e.neos - 1) {
     ientry = e.neos - 1;
-    eng = at(e.eng2, e.neos, irho);
+    eng = engn;
     eps = eng * rho;
   }
-  if (ientry < 1 || eng < at(e.eng2, 1, irho)) {
+  if (ientry < 1 || eng < eng1) {
     ientry = 1;
-    eng = at(e.eng2, 1, irho);
+    eng = eng1;
     eps = eng * rho;
   }
   // t(ientry) + (t(ientry+1) - t(ientry)) / (eng(ientry+1) - eng(ientry)) *
-  // (eng - eng(ientry)) for gamma, mu and T of density row ir: the three
-  // quotients share the denominator, so one exact shared reciprocal
+  // (eng - eng(ientry)) for gamma, mu and T of density row ir
   auto lin3 = [&](int ir, double& g3, double& m3, double& t3) {
-    const double e0 = at(e.eng2, ientry, ir);
-    const SharedDiv q(at(e.eng2, ientry + 1, ir) - e0);
-    const double de = eng - e0;
-    g3 = at(e.gam2, ientry, ir) + q(at(e.gam2, ientry + 1, ir) - at(e.gam2, ientry, ir)) * de;
-    m3 = at(e.muc2, ientry, ir) + q(at(e.muc2, ientry + 1, ir) - at(e.muc2, ientry, ir)) * de;
-    t3 = at(e.tk2, ientry, ir) + q(at(e.tk2, ientry + 1, ir) - at(e.tk2, ientry, ir)) * de;
+    const double2* p = reinterpret_cast<const double2*>(
+        e.pack + 8 * ((long long)(ir - 1) * e.neos + (ientry - 1)));
+    const double2 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3);
+    const double de = eng - a.x;
+    g3 = a.y + b.x * de;
+    m3 = b.y + c.x * de;
+    t3 = c.y + d.x * de;
   };
   lin3(irho, gam, m, tk);
-  if (!(e.rho[irho - 1] == e.rho[irhop - 1])) {
+  const double2 r3 = __ldg(row + 3);
+  if (r3.x != 0.0) {  // the next row has another density
     double gamp, mp, tkp;
-    lin3(irhop, gamp, mp, tkp);
-    const double slope = 1.0 / (e.rho[irhop - 1] - e.rho[irho - 1]) * (rho - e.rho[irho - 1]);
+    lin3(irho + 1, gamp, mp, tkp);
+    const double slope = r2.y * (rho - r2.x);
     gam = gam + (gamp - gam) * slope;
     m = m + (mp - m) * slope;
     tk = tk + (tkp - tk) * slope;
   }
 }
-
 
 // Loads of the stage inputs: through the read-only path when the planes stay
 // unchanged for the whole launch (one launch per stage), from L2 (cg) in the
@@ -229,15 +232,13 @@ __device__ __forceinline__ Raw load_raw(const StageArgs& a, const Place& p, int 
 // residual correction (exact).  The corrections are valid while the numerators'
 // exponents lie in their window; one check of all of them at the end, rather
 // than a branch per division, and false sends the caller to prim_ieee.
-// LIB: with the library's reciprocal and root (the flux_ang instances, which
-// spill; the short forms' chains side by side would add to it).
-template <int STAGE, bool LIB = false>
+template <int STAGE>
 __device__ __forceinline__ bool prim_fast(const Geom& g, const Cons& c, double v1, double v2,
                                           double v3, int nsrc, bool need_c, Prim& q, int rs = 0) {
   const bool is0 = stage_is0<STAGE>(rs);
   const double d = c.d;
   bool ok = den_fast_ok(d);
-  const double r = LIB ? (ok ? __drcp_rn(d) : 1.0) : rcp_fast(d);
+  const double r = rcp_fast(d);
   double E = c.E;
   if (is0) {
     // source(): E = max(E - K, eps) + K with K = half*|m|^2/rho, the same K each time
@@ -258,8 +259,7 @@ __device__ __forceinline__ bool prim_fast(const Geom& g, const Cons& c, double v
   if (need_c) {
     const double pn = q.p * g.gam;
     ok = ok && rad_fast_ok(pn);
-    const double qc = quot_fast(pn, d, r);
-    q.c = LIB ? sqrt(qc) : sqrt_fast(qc);
+    q.c = sqrt_fast(quot_fast(pn, d, r));
   }
   return ok;
 }
@@ -282,7 +282,7 @@ __device__ __forceinline__ Prim prim_ieee(double small_eps, double gm1, double g
   return q;
 }
 
-template <int STAGE, bool GRAV = false, bool TAB = false, bool ANG = false>
+template <int STAGE, bool GRAV = false, bool TAB = false>
 __device__ __forceinline__ Prim prim_of(const Geom& g, Raw r, int nsrc, double dth,
                                         bool need_c = true, int rs = 0,
                                         const EosDev* eos = nullptr) {
@@ -302,7 +302,7 @@ __device__ __forceinline__ Prim prim_of(const Geom& g, Raw r, int nsrc, double d
     q.p = eos_pressure(q.d, c.E, v1, v2, v3, g.gm1, g.small_eps);
     // the sound speed enters only the lambdas of cells whose face states are built
     q.c = need_c ? sqrt(qd(q.p * g.gam)) : 0.0;
-  } else if (!prim_fast<STAGE, ANG>(g, r.c, r.v1, r.v2, r.v3, nsrc, need_c && !TAB, q, rs)) {
+  } else if (!prim_fast<STAGE>(g, r.c, r.v1, r.v2, r.v3, nsrc, need_c && !TAB, q, rs)) {
     q = prim_ieee<STAGE>(g.small_eps, g.gm1, g.gam, r.c, r.v1, r.v2, r.v3, nsrc,
                          need_c && !TAB, rs);
   }
@@ -315,9 +315,9 @@ __device__ __forceinline__ Prim prim_of(const Geom& g, Raw r, int nsrc, double d
                      : at_least(r.c.E - kin_rho_u(q.d, r.v1, r.v2, r.v3), g.small_eps);
     double tk, m, gam;
     get_gamma2(*eos, eps, q.d, tk, m, gam);
-    q.p = (q.d * tk * g.rgas / m);
+    q.p = SharedDiv(m)(q.d * tk * g.rgas);
     q.g = gam;
-    q.c = need_c ? sqrt(q.p * gam / q.d) : 0.0;
+    q.c = need_c ? sound_of(q.p * gam, q.d) : 0.0;
   }
   return q;
 }
@@ -491,15 +491,16 @@ __device__ __forceinline__ void epi_ieee(const Geom& g, const double n[5], doubl
 template <bool POW2>
 __device__ __forceinline__ void epi_tab(const Geom& g, const EosDev& eos, const double n[5],
                                         double& u1, double& u2, double& u3, double& r0) {
-  u1 = n[1] / n[0];
-  u2 = n[2] / n[0];
-  u3 = n[3] / n[0];
-  const double E3 = source_energy(n[0], n[1], n[2], n[3], n[4], g.small_eps);
+  const SharedDiv qn(n[0]);
+  u1 = qn(n[1]);
+  u2 = qn(n[2]);
+  u3 = qn(n[3]);
+  const double E3 = source_energy_q(qn, n[1], n[2], n[3], n[4], g.small_eps);
   double eps = at_least(E3 - kin_rho_u(n[0], u1, u2, u3), g.small_eps);
   double tk, m, gam;
   get_gamma2(eos, eps, n[0], tk, m, gam);
-  const double p = (n[0] * tk * g.rgas / m);
-  r0 = courant_rate<POW2>(n[0], p, gam, u1, u2, u3, g.dx, g.dy, g.dz, g.idx, g.idy, g.idz);
+  const double p = SharedDiv(m)(n[0] * tk * g.rgas);
+  r0 = courant_rate_q<POW2>(qn, p, gam, u1, u2, u3, g.dx, g.dy, g.dz, g.idx, g.idy, g.idz);
 }
 
 // ------------------------------------------------------------------ stage kernel
@@ -630,7 +631,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
     return p;
   };
   auto prim_at = [&](const Raw& r, int x, int y) {
-    Prim q = prim_of<STAGE, GRAV, TAB, ANG>(g, r, nsrc, dth, true, rs, &a.eos);
+    Prim q = prim_of<STAGE, GRAV, TAB>(g, r, nsrc, dth, true, rs, &a.eos);
     // with flux_ang the momenta reconstructed are the transformed ones (the
     // sources leave the momenta alone)
     if (ANG) ang_to(g, x, y, r.c.m1, r.c.m2, q.rm, q.am);
@@ -1997,13 +1998,14 @@ cudaError_t fused_to_phase(const Geom& g, const double* X, int nsrc, PhaseArrays
   k_f2p_prims<<<nblk(g.ng), PB, 0, s>>>(g, a);
   return cudaGetLastError();
 }
-__global__ void k_log10_rows(const double* eng2, long long neos, int nr, double* out) {
+// the first value of each row record: log10 of the row's first energy, by the
+// device's log10 that the exact index takes
+__global__ void k_log10_rows(double* rows, int nr) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < nr) out[r] = log10(eng2[(long long)r * neos]);
+  if (r < nr) rows[8 * r] = log10(rows[8 * r + 2]);
 }
-cudaError_t eos_log_rows(const double* eng2, long long neos, int nr, double* out,
-                         cudaStream_t s) {
-  k_log10_rows<<<(nr + 127) / 128, 128, 0, s>>>(eng2, neos, nr, out);
+cudaError_t eos_log_rows(double* rows, int nr, cudaStream_t s) {
+  k_log10_rows<<<(nr + 127) / 128, 128, 0, s>>>(rows, nr);
   return cudaGetLastError();
 }
 __global__ void k_fill_const(double* a, long long n, double v) {

@@ -35,6 +35,13 @@ int bx_check_root(const double *q, unsigned long long n, unsigned long long nran
                   unsigned long long seed, int exp_range, unsigned long long *mismatches,
                   double *example);
 
+/* Self-check of the tabulated EOS's table index, (int)((log10(x) - low) / step), by
+ * the single-precision logarithm away from the steps' edges: n arguments at the
+ * edges of `steps` steps, off by 2^-1 to 2^-53 of themselves or not at all, against
+ * the double-precision form; returns the number that differ and one example. */
+int bx_check_log_steps(unsigned long long n, unsigned long long seed, double low, double step,
+                       int steps, unsigned long long *mismatches, double *example);
+
 #ifdef __cplusplus
 }
 #endif
