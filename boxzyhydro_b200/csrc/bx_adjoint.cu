@@ -114,7 +114,7 @@ __global__ void k_r1_prims(Geom g, int stage, const double* A, const double* B, 
   P[3 * n + i] = u3;
   P[4 * n + i] = p;
   P[5 * n + i] = e;
-  P[6 * n + i] = sqrt(qa(p * g.gam));
+  P[6 * n + i] = sound_of(p * g.gam, a.d);
 }
 
 // ---- conserved-variable VJP at cell (x,y,z) of a stage: gq holds the adjoints

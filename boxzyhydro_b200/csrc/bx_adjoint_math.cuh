@@ -47,7 +47,12 @@ __device__ __forceinline__ void hll_vjp(const FaceState& L, const FaceState& R, 
   }
   fl[4] = (sl[4] + pl) * vl;
   fr[4] = (sr[4] + pr) * vr;
-  const double cr = sqrt(gam * pr / dr), cl = sqrt(gam * pl / dl);
+  const double nr = gam * pr, nl = gam * pl;
+  double cr = sound_fast(nr, dr), cl = sound_fast(nl, dl);
+  if (!(den_fast_ok(dr) && den_fast_ok(dl) && rad_fast_ok(nr) && rad_fast_ok(nl))) {
+    cr = sound_ieee(nr, dr);
+    cl = sound_ieee(nl, dl);
+  }
   // ap = max(0, vr+cr, vl+cl), am = max(0, -(vr-cr), -(vl-cl)), evaluated as the forward
   const double a1 = vr + cr, a2 = vl + cl;
   const double b1 = -(vr - cr), b2 = -(vl - cl);
@@ -130,12 +135,15 @@ __device__ __forceinline__ void hll_vjp(const FaceState& L, const FaceState& R, 
 // the slope is zero)
 __device__ __forceinline__ double slope_and_sel(double c0, double c1, double c2, int& sel) {
   const double d1 = c1 - c0, d2 = c2 - c0, d3 = c2 - c1;
-  const double x1 = fabs(kTheta * d1), x2 = fabs(kHalf * d2), x3 = fabs(kTheta * d3);
-  const double m23 = fmin(x2, x3);
-  const double m = fmin(x1, m23);
-  const bool pos = (d1 > 0.0) && (d3 > 0.0), neg = (d1 < 0.0) && (d3 < 0.0);
-  sel = !(pos || neg) ? 0 : (x1 <= m23 ? 1 : (x2 <= x3 ? 2 : 3));
-  return pos ? m : (neg ? -m : 0.0);
+  const double x1 = kTheta * d1, x2 = kHalf * d2, x3 = kTheta * d3;
+  const bool two = fabs(x2) <= fabs(x3);
+  const double m23 = two ? x2 : x3;
+  const bool one = fabs(x1) <= fabs(m23);
+  const double m = one ? x1 : m23;
+  // d1 and d3 of one strict sign (slope3)
+  const bool take = (__double2hiint(d1) ^ __double2hiint(d3)) >= 0 && m != 0.0;
+  sel = !take ? 0 : (one ? 1 : (two ? 2 : 3));
+  return take ? m : 0.0;
 }
 
 }  // namespace bx
