@@ -174,25 +174,6 @@ __device__ __forceinline__ void cons_vjp_v(const Geom& g, int stage, const CvIn&
   gA[0] += grho;
 }
 
-// the same at (x,y,z) with the values read from memory (P at index pi)
-__device__ __forceinline__ void cons_vjp(const Geom& g, int stage, const double* P, long long pi,
-                                         const double* A, const double* B, int x, int y, int z,
-                                         const double gq[7], double gA[5], double gB[5]) {
-  const long long n = g.ng;
-  CvIn v;
-  v.rho = P[pi];
-  v.u[0] = P[n + pi]; v.u[1] = P[2 * n + pi]; v.u[2] = P[3 * n + pi];
-  v.p = P[4 * n + pi]; v.e = P[5 * n + pi]; v.cs = P[6 * n + pi];
-  v.aE = 0.0; v.bd = 1.0; v.bm[0] = v.bm[1] = v.bm[2] = 0.0;
-  if (stage == 1) {
-    const C5 a = aload(A, n, g, x, y, z);
-    const C5 b = aload(B, n, g, x, y, z);
-    v.aE = a.E;
-    v.bd = b.d; v.bm[0] = b.m1; v.bm[1] = b.m2; v.bm[2] = b.m3;
-  }
-  cons_vjp_v(g, stage, v, gq, gA, gB);
-}
-
 // ---- reverse of the faces of one direction, line by line.
 // A line is a row of cells along DIR at interior coordinates in the other
 // directions, from the ghost below the interior (lo-1) to the ghost above (hi);
@@ -223,22 +204,35 @@ __device__ __forceinline__ void cons_vjp(const Geom& g, int stage, const double*
 __host__ __device__ inline int rdir_x0(const Geom& g) { return g.ax0 & ~3; }
 
 struct RShape {
-  int NL, W, NQ, NS, NF, ND, nseg, threads;
-  size_t r1, r2, r3, r4, smem;  // region sizes in doubles; smem in bytes
+  int NL, W, nseg, threads;
+};
+
+// Shared memory of a block: planes with strides fixed at compile time by the
+// block size T, whatever the lines' length, so every plane of a phase is an
+// immediate offset (with the strides as run-time counts a third of the executed
+// instructions formed addresses: 1700-1910 per cell and direction, 500 of them
+// FP64).  With at most 16 lines a block holds T states, so T faces and MUSCL cells, T
+// + 32 primitives and T - 32 segment cells of y or z lines (at least 8 lines).
+template <int DIR>
+struct RMem {
+  static constexpr int T = DIR == 0 ? 128 : 256;
+  static constexpr int Q = T + 32, C = DIR == 0 ? 0 : T - 32;
+  // The primitives (to P2) and the HLL derivatives (from P3) share R3, the face
+  // states (to P3) and the MUSCL adjoints (from P4) share R2 and, the last of
+  // these, the scaled output adjoints' LM: 89 KB for y and z lines, whose two blocks
+  // leave L1 about 70 KB for the loads in flight (107 KB measured 45 against 38 us
+  // at 64^3, fewer instructions notwithstanding)
+  static constexpr int R3 = 0, LM = 12 * T, R2 = LM + 5 * T, PA = R2 + 20 * T, SEL = PA + 7 * C;
+  static_assert(7 * Q <= 12 * T, "the primitives fit the derivatives' place");
+  static constexpr size_t bytes = (size_t)SEL * sizeof(double) + T * sizeof(int);
 };
 
 static RShape rshape(int Lc, int wmax, int target) {
   RShape r{};
   r.nseg = (Lc + wmax - 1) / wmax;
   r.W = (Lc + r.nseg - 1) / r.nseg;
-  r.NQ = r.W + 6; r.NS = r.W + 4; r.NF = r.W + 3; r.ND = r.W + 2;
-  r.NL = std::max(1, target / r.NS);
-  r.threads = std::min(1024, ((r.NL * r.NS + 31) / 32) * 32);
-  r.r1 = (size_t)std::max(7 * r.NQ + 5 * r.NS, 13 * r.ND) * r.NL;
-  r.r2 = (size_t)21 * r.NS * r.NL;
-  r.r3 = (size_t)12 * r.NF * r.NL;
-  r.r4 = (size_t)7 * r.W * r.NL;  // PA of the segment, fetched while the block computes
-  r.smem = (r.r1 + r.r2 + r.r3 + r.r4) * sizeof(double) + (size_t)r.NS * r.NL * sizeof(int);
+  r.NL = std::min(16, std::max(1, target / (r.W + 4)));
+  r.threads = ((r.NL * (r.W + 4) + 31) / 32) * 32;
   return r;
 }
 
@@ -260,24 +254,18 @@ template <int DIR, bool POW2>
 __global__ void __launch_bounds__(DIR == 0 ? 128 : 256, DIR == 0 ? 4 : 2)
 k_rdir(Geom g, const double* P, const double* lamL, double lscale, double dt, double* PA,
        RShape sh) {
-  const int NL = sh.NL, W = sh.W, NQ = sh.NQ, NS = sh.NS, NF = sh.NF, ND = sh.ND;
+  const int NL = sh.NL, W = sh.W, NQ = W + 6, NS = W + 4, NF = W + 3, ND = W + 2;
+  using M = RMem<DIR>;
+  constexpr int T = M::T;  // plane stride of the states, faces and MUSCL cells
   extern __shared__ double sm[];
-  // d slope(c+o) / d q(c) by the selected argument sq of genminmod (1:
-  // theta*(c1-c0), 2: half*(c2-c0), 3: theta*(c2-c1), 0: none): row o+1, column
-  // sq; c is the slope's c0 (o = +1), c1 (o = 0) or c2 (o = -1)
-  __shared__ double kk_tab[12];
-  if (threadIdx.x < 12) {
-    const int o = (int)threadIdx.x / 4 - 1, sq = (int)threadIdx.x % 4;
-    kk_tab[threadIdx.x] = o == 1 ? (sq == 1 ? -kTheta : (sq == 2 ? -kHalf : 0.0))
-                        : o == 0 ? (sq == 1 ? kTheta : (sq == 3 ? -kTheta : 0.0))
-                                 : (sq == 2 ? kHalf : (sq == 3 ? kTheta : 0.0));
-  }
-  double* r1 = sm;
-  double* r2 = sm + sh.r1;
-  double* r3 = r2 + sh.r2;
-  double* pa_s = r3 + sh.r3;  // [7][NL*W]
-  int* sel_s = reinterpret_cast<int*>(pa_s + sh.r4);
-  double* lm_s = r1 + 7 * NL * NQ;  // lives in r1 beside the primitives until P4
+  double* const r1 = sm + M::R3;    // [7][Q] primitives
+  double* const r3 = sm + M::R3;    // [12][T] HLL derivatives
+  double* const lm_s = sm + M::LM;  // [5][T] scaled output adjoints
+  double* const r2 = sm + M::R2;    // [20][T] minus and plus states, slopes, hm, hp
+  // the adjoints of P4: the cell's own (0-6) and of its slopes (7-12)
+  auto ad = [&](int q) -> double* { return q < 12 ? r2 + q * T : lm_s; };
+  double* const pa_s = sm + M::PA;  // [7][C]
+  int* const sel_s = reinterpret_cast<int*>(sm + M::SEL);
   const long long n = g.ng;
   const int zlo = g.threed ? g.az0 : 0, zhi = g.threed ? g.az1 : g.nz;
   const int nyi = g.ay1 - g.ay0, nzi = zhi - zlo;
@@ -337,7 +325,8 @@ k_rdir(Geom g, const double* P, const double* lamL, double lscale, double dt, do
       if (!valid(c) || first(c)) continue;
       const long long i = lb + c * st;
       const int kp = rsx<DIR>(l, j, W, NL);
-      for (int q = 0; q < 7; ++q) cp_async8(pa_s + q * NL * W + kp, PA + q * n + i);
+#pragma unroll
+      for (int q = 0; q < 7; ++q) cp_async8(pa_s + q * M::C + kp, PA + q * n + i);
     }
     cp_async_commit();
   }
@@ -349,15 +338,18 @@ k_rdir(Geom g, const double* P, const double* lamL, double lscale, double dt, do
     const int k = rsx<DIR>(l, j, NQ, NL);
     const long long i = lb + c * st;
     if (ok && valid(c)) {
-      for (int q = 0; q < 7; ++q) r1[q * NL * NQ + k] = P[q * n + i];
+#pragma unroll
+      for (int q = 0; q < 7; ++q) r1[q * M::Q + k] = P[q * n + i];
     } else {
-      for (int q = 0; q < 7; ++q) r1[q * NL * NQ + k] = 1.0;
+#pragma unroll
+      for (int q = 0; q < 7; ++q) r1[q * M::Q + k] = 1.0;
     }
     // scaled adjoints of the interior cells of [s0-2, s0+W+2) (zero elsewhere)
     if (j >= 1 && j <= NS) {
       const int kl = rsx<DIR>(l, j - 1, NS, NL);
       const bool in = ok && inner(c);
-      for (int q = 0; q < 5; ++q) lm_s[q * NL * NS + kl] = in ? lscale * lamL[q * n + i] : 0.0;
+#pragma unroll
+      for (int q = 0; q < 5; ++q) lm_s[q * T + kl] = in ? lscale * lamL[q * n + i] : 0.0;
     }
   }
   __syncthreads();
@@ -367,14 +359,14 @@ k_rdir(Geom g, const double* P, const double* lamL, double lscale, double dt, do
     const int k = rsx<DIR>(l, j, NS, NL);
     auto qv = [&](int jj) {
       const int kk = rsx<DIR>(l, jj, NQ, NL);
-      return Prim{r1[kk], r1[NL * NQ + kk], r1[2 * NL * NQ + kk], r1[3 * NL * NQ + kk],
-                  r1[4 * NL * NQ + kk], r1[5 * NL * NQ + kk], r1[6 * NL * NQ + kk]};
+      return Prim{r1[kk], r1[M::Q + kk], r1[2 * M::Q + kk], r1[3 * M::Q + kk],
+                  r1[4 * M::Q + kk], r1[5 * M::Q + kk], r1[6 * M::Q + kk]};
     };
     const Prim qc = qv(j + 1);
     FaceState mi, pl;
     double sl[6] = {0, 0, 0, 0, 0, 0};
     int sel = 0;
-    double hm = 0.0, hp = 0.0, flg = 0.0;
+    double hm = 0.0, hp = 0.0;
     if (inner(c)) {
       const Prim qm = qv(j), qp = qv(j + 2);
       const double a0[6] = {qm.d, qm.u1, qm.u2, qm.u3, qm.p, qm.e};
@@ -384,7 +376,10 @@ k_rdir(Geom g, const double* P, const double* lamL, double lscale, double dt, do
       for (int q = 0; q < 6; ++q) {
         int sq;
         sl[q] = slope_and_sel(a0[q], a1[q], a2[q], sq);
-        sel |= sq << (2 * q);
+        // which of the slope's cells its selected argument reads (P5): bit q, the
+        // one below (sel 1 or 2), 6 + q and 12 + q the cell itself (1: plus, 3: minus),
+        // 18 + q the one above (2 or 3); 24 + q, half of c2 - c0 (2)
+        sel |= (sq == 1 ? 0x41 : sq == 2 ? 0x1040001 : sq == 3 ? 0x41000 : 0) << q;
       }
       const double ud = DIR == 0 ? qc.u1 : DIR == 1 ? qc.u2 : qc.u3;
       muscl_states<POW2>(qc, ud, sl[0], sl[1], sl[2], sl[3], sl[4], sl[5], dt, ds, ids, mi, pl);
@@ -393,22 +388,20 @@ k_rdir(Geom g, const double* P, const double* lamL, double lscale, double dt, do
       else { lp = cdiv(lp, ds, ids); lm = cdiv(lm, ds, ids); }
       hm = kHalf * (-1.0 - lm);
       hp = kHalf * (1.0 - lp);
-      flg = (ud + qc.c > 0.0 ? 1.0 : 0.0) + (ud - qc.c < 0.0 ? 2.0 : 0.0);
+      sel |= (ud + qc.c > 0.0 ? 1 << 30 : 0) | (ud - qc.c < 0.0 ? (int)(1u << 31) : 0);
     } else {
       ghost_states(qc, mi, pl);
     }
-    const int M = NL * NS;
     const double mv[6] = {mi.d, mi.u1, mi.u2, mi.u3, mi.p, mi.e};
     const double pv[6] = {pl.d, pl.u1, pl.u2, pl.u3, pl.p, pl.e};
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
-      r2[q * M + k] = mv[q];
-      r2[(6 + q) * M + k] = pv[q];
-      r2[(12 + q) * M + k] = sl[q];
+      r2[q * T + k] = mv[q];
+      r2[(6 + q) * T + k] = pv[q];
+      r2[(12 + q) * T + k] = sl[q];
     }
-    r2[18 * M + k] = hm;
-    r2[19 * M + k] = hp;
-    r2[20 * M + k] = flg;
+    r2[18 * T + k] = hm;
+    r2[19 * T + k] = hp;
     sel_s[k] = sel;
   }
   __syncthreads();
@@ -417,64 +410,64 @@ k_rdir(Geom g, const double* P, const double* lamL, double lscale, double dt, do
     const int c = s0 - 1 + j;
     const bool ok = lok;
     const int k = rsx<DIR>(l, j, NF, NL);
-    const int M3 = NL * NF;
     if (!(ok && c >= lo && c <= hi)) {
-      for (int q = 0; q < 12; ++q) r3[q * M3 + k] = 0.0;
+#pragma unroll
+      for (int q = 0; q < 12; ++q) r3[q * T + k] = 0.0;
       continue;
     }
-    const int M = NL * NS;
     const int kl = rsx<DIR>(l, j, NS, NL), kr = rsx<DIR>(l, j + 1, NS, NL);
-    const FaceState L{r2[6 * M + kl], r2[7 * M + kl], r2[8 * M + kl], r2[9 * M + kl],
-                      r2[10 * M + kl], r2[11 * M + kl]};
-    const FaceState R{r2[kr], r2[M + kr], r2[2 * M + kr], r2[3 * M + kr], r2[4 * M + kr],
-                      r2[5 * M + kr]};
+    const FaceState L{r2[6 * T + kl], r2[7 * T + kl], r2[8 * T + kl], r2[9 * T + kl],
+                      r2[10 * T + kl], r2[11 * T + kl]};
+    const FaceState R{r2[kr], r2[T + kr], r2[2 * T + kr], r2[3 * T + kr], r2[4 * T + kr],
+                      r2[5 * T + kr]};
     double gF[5];
 #pragma unroll
-    for (int q = 0; q < 5; ++q) gF[q] = coef * (lm_s[q * NL * NS + kl] - lm_s[q * NL * NS + kr]);
+    for (int q = 0; q < 5; ++q) gF[q] = coef * (lm_s[q * T + kl] - lm_s[q * T + kr]);
     FS6 gL, gR;
     hll_vjp<DIR>(L, R, g.gam, gF, gL, gR);
     const double a[12] = {gL.d, gL.u1, gL.u2, gL.u3, gL.p, gL.e,
                           gR.d, gR.u1, gR.u2, gR.u3, gR.p, gR.e};
 #pragma unroll
-    for (int q = 0; q < 12; ++q) r3[q * M3 + k] = a[q];
+    for (int q = 0; q < 12; ++q) r3[q * T + k] = a[q];
   }
   __syncthreads();
-  // P4: MUSCL adjoint per cell c = s0-1+j (into r1: DQ planes 0-6, LS planes 7-12)
+  // P4: MUSCL adjoint per cell c = s0-1+j (own adjoints, and those of its slopes
+  // times their selected argument's factor)
   for (int j = j0; j < ND && lane; j += TPL) {
     const int c = s0 - 1 + j;
     const int k = rsx<DIR>(l, j, ND, NL);
-    const int M1 = NL * ND, M = NL * NS, M3 = NL * NF;
     double lq[7] = {0, 0, 0, 0, 0, 0, 0}, ls[6] = {0, 0, 0, 0, 0, 0};
     if (valid(c)) {
       const int kf0 = rsx<DIR>(l, j, NF, NL), kf1 = rsx<DIR>(l, j + 1, NF, NL);
       double gm[6], gp[6];
 #pragma unroll
       for (int q = 0; q < 6; ++q) {
-        gm[q] = r3[(6 + q) * M3 + kf0];  // minus state of c: high side of face (c-1, c)
-        gp[q] = r3[q * M3 + kf1];        // plus state of c: low side of face (c, c+1)
+        gm[q] = r3[(6 + q) * T + kf0];   // minus state of c: high side of face (c-1, c)
+        gp[q] = r3[q * T + kf1];         // plus state of c: low side of face (c, c+1)
         lq[q] = gm[q] + gp[q];
       }
       if (inner(c)) {
         const int ks = rsx<DIR>(l, j + 1, NS, NL);
-        const double hm = r2[18 * M + ks], hp = r2[19 * M + ks];
-        const int flg = (int)r2[20 * M + ks];
+        const double hm = r2[18 * T + ks], hp = r2[19 * T + ks];
+        const int sel = sel_s[ks];
         double ghm = 0.0, ghp = 0.0;
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
-          const double sq = r2[(12 + q) * M + ks];
-          ls[q] = hm * gm[q] + hp * gp[q];
+          const double sq = r2[(12 + q) * T + ks];
+          // times the selected argument's factor: what the slope's cells get, by sign
+          ls[q] = (sel >> (24 + q) & 1 ? kHalf : kTheta) * (hm * gm[q] + hp * gp[q]);
           ghm += sq * gm[q];
           ghp += sq * gp[q];
         }
         const double glm = -kHalf * ghm, glp = -kHalf * ghp;
-        if (flg & 1) { lq[1 + DIR] += glp * rr; lq[6] += glp * rr; }
-        if (flg & 2) { lq[1 + DIR] += glm * rr; lq[6] -= glm * rr; }
+        if (sel & 1 << 30) { lq[1 + DIR] += glp * rr; lq[6] += glp * rr; }
+        if (sel < 0) { lq[1 + DIR] += glm * rr; lq[6] -= glm * rr; }
       }
     }
 #pragma unroll
-    for (int q = 0; q < 7; ++q) r1[q * M1 + k] = lq[q];
+    for (int q = 0; q < 7; ++q) ad(q)[k] = lq[q];
 #pragma unroll
-    for (int q = 0; q < 6; ++q) r1[(7 + q) * M1 + k] = ls[q];
+    for (int q = 0; q < 6; ++q) ad(7 + q)[k] = ls[q];
   }
   __syncthreads();
   // P5: gather and accumulate
@@ -487,19 +480,32 @@ k_rdir(Geom g, const double* P, const double* lamL, double lscale, double dt, do
     if (!valid(c)) continue;
     const long long b = lb;
     const int kp = rsx<DIR>(l, j, W, NL);
-    const int M1 = NL * ND;
     const int kc = rsx<DIR>(l, j + 1, ND, NL);
     double acc[7];
 #pragma unroll
-    for (int q = 0; q < 7; ++q) acc[q] = r1[q * M1 + kc];
-#pragma unroll
-    for (int o = -1; o <= 1; ++o) {
-      if (!inner(c + o)) continue;
-      const int sel = sel_s[rsx<DIR>(l, j + 2 + o, NS, NL)];
-      const int kn = rsx<DIR>(l, j + 1 + o, ND, NL);
+    for (int q = 0; q < 7; ++q) acc[q] = ad(q)[kc];
+    // the slopes of the cells below, here and above, where their selected argument
+    // reads this one
+    if (inner(c - 1)) {
+      const int sel = sel_s[rsx<DIR>(l, j + 1, NS, NL)], kn = rsx<DIR>(l, j, ND, NL);
 #pragma unroll
       for (int q = 0; q < 6; ++q)
-        acc[q] += kk_tab[(o + 1) * 4 + ((sel >> (2 * q)) & 3)] * r1[(7 + q) * M1 + kn];
+        if (sel & 1 << (18 + q)) acc[q] += ad(7 + q)[kn];
+    }
+    if (inner(c)) {
+      const int sel = sel_s[rsx<DIR>(l, j + 2, NS, NL)];
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        const double v = ad(7 + q)[kc];
+        if (sel & 1 << (6 + q)) acc[q] += v;
+        if (sel & 1 << (12 + q)) acc[q] -= v;
+      }
+    }
+    if (inner(c + 1)) {
+      const int sel = sel_s[rsx<DIR>(l, j + 3, NS, NL)], kn = rsx<DIR>(l, j + 2, ND, NL);
+#pragma unroll
+      for (int q = 0; q < 6; ++q)
+        if (sel & 1 << q) acc[q] -= ad(7 + q)[kn];
     }
     const long long i = b + c * st;
     if (first(c)) {
@@ -507,7 +513,7 @@ k_rdir(Geom g, const double* P, const double* lamL, double lscale, double dt, do
       for (int q = 0; q < 7; ++q) PA[q * n + i] = acc[q];
     } else {
 #pragma unroll
-      for (int q = 0; q < 7; ++q) PA[q * n + i] = pa_s[q * NL * W + kp] + acc[q];
+      for (int q = 0; q < 7; ++q) PA[q * n + i] = pa_s[q * M::C + kp] + acc[q];
     }
   }
 }
@@ -519,51 +525,25 @@ k_rdir(Geom g, const double* P, const double* lamL, double lscale, double dt, do
 //           o2 <- adjoint of C0' so far = (lin/2 + a_B) + o1;
 //  stage 0 (lin = adjoint of C0' so far): o1 <- (lin + a_A) + a_B, then through
 //           the nsrc sources of X (source.f90:176-182); ghost entries of o1 zero.
-// conserved adjoints of the face ghosts next to interior cell (x,y,z) whose donor
-// it is, added to a (kept out of line: only boundary cells take it)
-template <int STAGE>
-__device__ __noinline__ void ghost_fold(const Geom& g, const double* SA, const double* SB,
-                                        const double* P, const double* PA, int x, int y, int z,
-                                        long long i, double a[10]) {
-  const long long n = g.ng;
-  const int ndir = g.threed ? 3 : 2;
-  const int lo[3] = {g.ax0, g.ay0, g.az0}, hi[3] = {g.ax1, g.ay1, g.az1};
-  const int c[3] = {x, y, z};
-  double gq[7], gA[5], gB[5];
-  for (int dir = 0; dir < ndir; ++dir) {
-    const long long st = dir == 0 ? 1 : dir == 1 ? g.sy : g.sz;
-    for (int side = 0; side < 2; ++side) {
-      // the face ghost next to this cell (lo-1 or hi), whose donor is this cell
-      if (c[dir] != (side == 0 ? lo[dir] : hi[dir] - 1)) continue;
-      const int gc = side == 0 ? lo[dir] - 1 : hi[dir];
-      const long long gi = i + (long long)(gc - c[dir]) * st;
-      const bool flip = g.wall[2 * dir + side] != 0;
-      for (int q = 0; q < 7; ++q) gq[q] = PA[q * n + gi];
-      int gx = x, gy = y, gz = z;
-      if (dir == 0) gx = gc; else if (dir == 1) gy = gc; else gz = gc;
-      cons_vjp(g, STAGE, P, gi, SA, SB, gx, gy, gz, gq, gA, gB);
-      for (int q = 0; q < 5; ++q) {
-        const bool neg = flip && q == 1 + dir;
-        a[q] += neg ? -gA[q] : gA[q];
-        a[5 + q] += neg ? -gB[q] : gB[q];
-      }
-    }
-  }
-}
-
-// grid over interior cells: x threads by (y, z) blocks.  Writes interior entries
-// only (the ghost entries of the adjoint planes stay zero).
+// Writes interior entries only (the ghost entries of the adjoint planes stay zero).
+// Bound by the loads in flight (0.2 KB a cell).  Measured at 64^3, stage 1 / 0: 40 /
+// 32 us as two launches with the fold out of line, its arrays through local memory
+// (23 local stores for every cell) and every ghost's values loaded anew; 28 / 24 in
+// one launch; 19 / 17 with the fold in line on the cell's own values.
 template <int STAGE>
 __global__ void k_rcell(Geom g, const double* SA, const double* SB, const double* P,
                         const double* PA, const double* lin, double* o1, double* o2,
-                        const double* X, int nsrc, int xedge) {
-  // xedge = 0: the columns between the two x-edge columns (every warp takes the
-  // ghost path together or not at all); xedge = 1: the two x-edge columns
+                        const double* X, int nsrc, int nbx, unsigned nedge) {
+  // the first nedge blocks take the two x-edge columns, whose cells all fold
+  // ghosts (their long chains start first); the others, nbx blocks a row, the
+  // columns between them, where a warp takes the ghost path together or not at
+  // all.  One launch: the x edges as a launch of their own after the rest took as
+  // long again at 64^3.
   int x, y, z;
-  if (xedge) {
+  const int nyi = g.ay1 - g.ay0, nzi = g.threed ? g.az1 - g.az0 : g.nz;
+  if (blockIdx.x < nedge) {
     // one thread per x-edge cell: t = side + 2 (y + nyi z)
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const int nyi = g.ay1 - g.ay0, nzi = g.threed ? g.az1 - g.az0 : g.nz;
     if (t >= 2ll * nyi * nzi) return;
     const int side = (int)(t & 1);
     if (side == 1 && g.ax1 - 1 == g.ax0) return;
@@ -571,16 +551,18 @@ __global__ void k_rcell(Geom g, const double* SA, const double* SB, const double
     y = g.ay0 + (int)((t >> 1) % nyi);
     z = (g.threed ? g.az0 : 0) + (int)((t >> 1) / nyi);
   } else {
-    x = g.ax0 + 1 + blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned b = blockIdx.x - nedge, row = b / (unsigned)nbx;
+    x = g.ax0 + 1 + (int)(b % (unsigned)nbx) * blockDim.x + threadIdx.x;
     if (x >= g.ax1 - 1) return;
-    y = g.ay0 + blockIdx.y;
-    z = (g.threed ? g.az0 : 0) + blockIdx.z;
+    y = g.ay0 + (int)(row % (unsigned)nyi);
+    z = (g.threed ? g.az0 : 0) + (int)(row / (unsigned)nyi);
   }
   const long long i = x + (long long)y * g.sy + (long long)z * g.sz;
   const long long n = g.ng;
   // every load of the cell first (an interior cell is its own donor)
   double gq[7], a[10], gA[5], gB[5], li[5], xs[5];
   CvIn v;
+#pragma unroll
   for (int q = 0; q < 7; ++q) gq[q] = __ldg(PA + q * n + i);
   v.rho = __ldg(P + i);
   v.u[0] = __ldg(P + n + i); v.u[1] = __ldg(P + 2 * n + i); v.u[2] = __ldg(P + 3 * n + i);
@@ -599,11 +581,37 @@ __global__ void k_rcell(Geom g, const double* SA, const double* SB, const double
   const bool edge = x == g.ax0 || x == g.ax1 - 1 || y == g.ay0 || y == g.ay1 - 1 ||
                     (g.threed && (z == g.az0 || z == g.az1 - 1));
   if (edge) {
-    // the fold takes its array through memory; only the edge cells pay for that
-    double e[10];
-    for (int q = 0; q < 10; ++q) e[q] = a[q];
-    ghost_fold<STAGE>(g, SA, SB, P, PA, x, y, z, i, e);
-    for (int q = 0; q < 10; ++q) a[q] = e[q];
+    // the conserved adjoints of the face ghosts next to the cell, whose donor it is:
+    // their values are the cell's own, the normal components reversed at a wall,
+    // so a ghost's primitive adjoints are all there is to load
+#pragma unroll 1
+    for (int k = 0; k < (g.threed ? 6 : 4); ++k) {
+      const int dir = k >> 1, side = k & 1;
+      const int c = dir == 0 ? x : dir == 1 ? y : z;
+      const int lo = dir == 0 ? g.ax0 : dir == 1 ? g.ay0 : g.az0;
+      const int hi = dir == 0 ? g.ax1 : dir == 1 ? g.ay1 : g.az1;
+      if (c != (side ? hi - 1 : lo)) continue;
+      const long long st = dir == 0 ? 1 : dir == 1 ? g.sy : g.sz;
+      const long long gi = side ? i + st : i - st;
+      const bool flip = g.wall[k] != 0;
+      CvIn w = v;
+      double hq[7];
+#pragma unroll
+      for (int q = 0; q < 7; ++q) hq[q] = __ldg(PA + q * n + gi);
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        if (flip && q == dir) {
+          w.u[q] = -w.u[q];
+          w.bm[q] = -w.bm[q];
+        }
+      cons_vjp_v(g, STAGE, w, hq, gA, gB);
+#pragma unroll
+      for (int q = 0; q < 5; ++q) {
+        const bool neg = flip && q == 1 + dir;
+        a[q] += neg ? -gA[q] : gA[q];
+        a[5 + q] += neg ? -gB[q] : gB[q];
+      }
+    }
   }
   if constexpr (STAGE == 1) {
     for (int q = 0; q < 5; ++q) {
@@ -1172,11 +1180,11 @@ static cudaError_t launch_rdir(const Geom& g, const double* P, const double* lam
   // x lines run along contiguous memory: long segments; y/z lines: 8 lines of
   // adjacent x per block (coalesced), short segments
   const RShape sh = DIR == 0 ? rshape(hi - lo + 2, 60, 128) : rshape(hi - lo + 2, 28, 256);
-  cudaError_t e = ensure_dyn_smem((const void*)k_rdir<DIR, POW2>, sh.smem);
+  cudaError_t e = ensure_dyn_smem((const void*)k_rdir<DIR, POW2>, RMem<DIR>::bytes);
   if (e != cudaSuccess) return e;
   const long long ngrp = (nlines + sh.NL - 1) / sh.NL;
   const dim3 grid((unsigned)(ngrp * sh.nseg));
-  k_rdir<DIR, POW2><<<grid, sh.threads, sh.smem, s>>>(g, P, lamL, lscale, dt, PA, sh);
+  k_rdir<DIR, POW2><<<grid, sh.threads, RMem<DIR>::bytes, s>>>(g, P, lamL, lscale, dt, PA, sh);
   return cudaGetLastError();
 }
 
@@ -1201,20 +1209,17 @@ static int rev_stage(bx_adj* A, int stage, const double* SA, const double* SB, c
   k_r1_prims<<<pgrid, tp, 0, s>>>(g, stage, SA, SB, A->P);
   // interior cells
   const int nxm = std::max(1, g.ax1 - g.ax0 - 2), tc = std::min(256, ((nxm + 31) / 32) * 32);
-  const dim3 cgrid((unsigned)((nxm + tc - 1) / tc), (unsigned)(g.ay1 - g.ay0),
-                   (unsigned)(g.threed ? g.az1 - g.az0 : g.nz));
-  const long long nedge = 2ll * cgrid.y * cgrid.z;
-  const dim3 egrid((unsigned)((nedge + 127) / 128));
+  const int nbx = (nxm + tc - 1) / tc;
+  const long long rows = (long long)(g.ay1 - g.ay0) * (g.threed ? g.az1 - g.az0 : g.nz);
+  const unsigned nedge = (unsigned)((2 * rows + tc - 1) / tc);
+  const unsigned cgrid = nedge + (unsigned)(nbx * rows);  // below 2^31: the grid is
   ACK(launch_rdir<0>(g, A->P, lamL, lscale, dt, A->PA, s));
   ACK(launch_rdir<1>(g, A->P, lamL, lscale, dt, A->PA, s));
   if (g.threed) ACK(launch_rdir<2>(g, A->P, lamL, lscale, dt, A->PA, s));
-  if (stage == 1) {
-    k_rcell<1><<<cgrid, tc, 0, s>>>(g, SA, SB, A->P, A->PA, lin, o1, o2, X, nsrc, 0);
-    k_rcell<1><<<egrid, 128, 0, s>>>(g, SA, SB, A->P, A->PA, lin, o1, o2, X, nsrc, 1);
-  } else {
-    k_rcell<0><<<cgrid, tc, 0, s>>>(g, SA, SB, A->P, A->PA, lin, o1, o2, X, nsrc, 0);
-    k_rcell<0><<<egrid, 128, 0, s>>>(g, SA, SB, A->P, A->PA, lin, o1, o2, X, nsrc, 1);
-  }
+  if (stage == 1)
+    k_rcell<1><<<cgrid, tc, 0, s>>>(g, SA, SB, A->P, A->PA, lin, o1, o2, X, nsrc, nbx, nedge);
+  else
+    k_rcell<0><<<cgrid, tc, 0, s>>>(g, SA, SB, A->P, A->PA, lin, o1, o2, X, nsrc, nbx, nedge);
   ACK(cudaGetLastError());
   return BX_OK;
 }
