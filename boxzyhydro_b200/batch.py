@@ -3,7 +3,7 @@
 The reference advances one grid per process.  `Batch` advances many grids at
 once -- each with its own size, gamma, CFL number, dt and clock -- with the same
 stage kernels as `Hydro`, so every box evolves exactly as it would alone; a run
-of n steps is one CUDA graph launch (four kernels per step, or one persistent
+of n steps is one CUDA graph launch (three kernels per step, or one persistent
 kernel for the whole run).
 """
 from __future__ import annotations
@@ -69,7 +69,7 @@ class Batch:
         self._c(lib().bx_batch_run(self._h, int(nsteps), float(endtime), 1 if graph else 0))
 
     def set_persistent(self, enable=True):
-        """One launch per run (a queue of step/stage/tile items) instead of four
+        """One launch per run (a queue of step/stage/tile items) instead of three
         launches per step; the same results."""
         self._c(lib().bx_batch_set_persistent(self._h, 1 if enable else 0))
 
@@ -91,7 +91,7 @@ class Batch:
         return bool(e.value)
 
     def autotune(self, reps=2):
-        """Pick the ensemble's tile shape and depth, then the launch form (four
+        """Pick the ensemble's tile shape and depth, then the launch form (three
         launches per step or one persistent launch), by timing trial steps from the
         current states (left unchanged): returns (depth, ms per step); depth 0 is
         the default rule, >= 2**30 whole box depths; `tile_shape` and `persistent`

@@ -693,7 +693,6 @@ __global__ void k_set_clock(Ctrl* c, double dt, int active) {
   c->dt = dt;
   c->active = active;
 }
-__global__ void k_record_dt(const Ctrl* c, double* dts, long long k) { dts[k] = c->dt; }
 
 // ---- frozen-branch forward.  A base state and a perturbed state advance
 // together through the fused step (dt frozen at the recorded sequence); the
@@ -1743,8 +1742,7 @@ int bx_adj_forward(bx_adj* A, const double* cons0, double* consT, int32_t frozen
     if (given_dt) {
       k_set_clock<<<1, 1, 0, s>>>(h->d_ctrl, A->dts[k], 1);
     } else {
-      ACK(launch_dt(h->d_ctrl, 1, s));
-      k_record_dt<<<1, 1, 0, s>>>(h->d_ctrl, A->d_dts, k);
+      if (k == 0) ACK(launch_begin_run(h->d_ctrl, A->d_dts, s));
     }
     a.X = cur;
     a.out = (!frozen && A->c1pool) ? A->c1pool + k * n5 : A->W1;
@@ -1752,7 +1750,8 @@ int bx_adj_forward(bx_adj* A, const double* cons0, double* consT, int32_t frozen
     a.Y = a.out;
     a.out = out;
     ACK(launch_stage(1, g.pow2 ? 1 : 0, g.threed != 0, a, h->ntiles, s));
-    if (!given_dt) ACK(launch_end(h->d_ctrl, 1, s));
+    if (!given_dt)
+      ACK(launch_next_run(h->d_ctrl, k + 1 < A->nsteps ? A->d_dts + k + 1 : nullptr, s));
     if (hb >= 0) {
       ACK(cudaEventRecord(A->uev[hb], s));
       ACK(cudaStreamWaitEvent(A->cstream, A->uev[hb], 0));

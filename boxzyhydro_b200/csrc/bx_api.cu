@@ -237,6 +237,7 @@ int bx_destroy(bx_handle* h) {
   cudaFree(h->d_tiles);
   cudaFree(h->d_ctrl);
   if (h->h_ctrl) cudaFreeHost(h->h_ctrl);
+  if (h->ev_copied) cudaEventDestroy(h->ev_copied);
   for (int k = 0; k < 3; ++k)
     if (h->ev[k]) cudaEventDestroy(h->ev[k]);
   if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
@@ -423,7 +424,7 @@ int bx_set_clock(bx_handle* h, double time, double dtold, int64_t step) {
 
 int bx_get_clock(bx_handle* h, double* time, double* dt, double* dtold, int64_t* step) {
   CHECK_H();
-  if (int r = pull_clock(h)) return r;
+  // every call that moves the clock leaves the host's copy current
   if (time) *time = h->clock.time;
   if (dt) *dt = h->clock.dt;
   if (dtold) *dtold = h->clock.dtold;
@@ -635,8 +636,11 @@ int bx_set_phi(bx_handle* h, const double* phi) {
   if (!h->pa.gforce) CK(dalloc((void**)&h->pa.gforce, 3 * n * sizeof(double)));
   double* tmp = staging(h);
   CK(cudaMemcpyAsync(tmp, phi, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  // the caller may reuse phi once the copy is done; calc_gforce need not be
+  if (!h->ev_copied) CK(cudaEventCreateWithFlags(&h->ev_copied, cudaEventDisableTiming));
+  CK(cudaEventRecord(h->ev_copied, h->stream));
   CK(phase_calc_gforce(h->g, tmp, h->pa.gforce, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
+  CK(cudaEventSynchronize(h->ev_copied));
   h->gforce_set = true;
   update_eligible(h);
   return BX_OK;
@@ -797,8 +801,10 @@ static int after_fused(bx_handle* h, const Ctrl& before, int32_t* ran, bool time
     h->grav_step = h->gforce_set;
     h->p_saved = false;
     h->nsrc = h->gforce_set ? 1 : 2;
-    h->clock.flags = 0;
-    if (int r = push_clock(h)) return r;
+    if (f) {  // (otherwise the device's block is the mirror's already)
+      h->clock.flags = 0;
+      if (int r = push_clock(h)) return r;
+    }
     h->last_path = 1;
     if (ran) *ran = 1;
     return BX_OK;
@@ -1240,11 +1246,15 @@ static int fused_run(bx_handle* h, double endtime, int64_t nsteps, int64_t* take
   const Geom& g = h->g;
   cudaStream_t s = h->stream;
   const int K = (int)std::min<int64_t>(nsteps, kRunChunk);
-  h->clock.endtime = endtime;
-  h->clock.flags = 0;
-  h->clock.tripped = 0;
-  h->clock.run_step = 0;
-  if (int r = push_clock(h)) return r;
+  // the device's control block is the mirror's after every call, but for flags that
+  // state() with the tables may raise while the arrays are rebuilt for a download
+  if (h->clock.endtime != endtime || h->clock.flags || h->clock.tripped || g.tab) {
+    h->clock.endtime = endtime;
+    h->clock.flags = 0;
+    h->clock.tripped = 0;
+    h->clock.run_step = 0;
+    if (int r = push_clock(h)) return r;
+  }
   const long long step0 = h->clock.step;
   const int cur0 = h->cur;
   StageArgs a{};
@@ -1259,8 +1269,8 @@ static int fused_run(bx_handle* h, double endtime, int64_t nsteps, int64_t* take
   const bool p2 = g.pow2 != 0, t3 = g.threed != 0;
   auto enqueue = [&]() -> cudaError_t {
     int cur = cur0;
+    cudaError_t e = launch_dt_batch(h->d_ctrl, 1, s);
     for (int k = 0; k < K; ++k) {
-      cudaError_t e = launch_dt_batch(h->d_ctrl, 1, s);
       a.nsrc = k == 0 ? h->nsrc : (h->gforce_set ? 1 : 2);
       a.X = h->buf[cur];
       a.Y = nullptr;
@@ -1269,7 +1279,8 @@ static int fused_run(bx_handle* h, double endtime, int64_t nsteps, int64_t* take
       a.Y = h->buf[(cur + 1) % 3];
       a.out = h->buf[(cur + 2) % 3];
       if (e == cudaSuccess) e = launch_stage(1, p2, t3, a, h->ntiles, s, h->shape);
-      if (e == cudaSuccess) e = launch_end_batch(h->d_ctrl, 1, s);
+      if (e == cudaSuccess)
+        e = k + 1 < K ? launch_next_batch(h->d_ctrl, 1, s) : launch_end_batch(h->d_ctrl, 1, s);
       if (e != cudaSuccess) return e;
       cur = (cur + 2) % 3;
     }
@@ -1294,7 +1305,7 @@ static int fused_run(bx_handle* h, double endtime, int64_t nsteps, int64_t* take
   } else {
     CK(enqueue());
   }
-  h->launches += 4 * K;
+  h->launches += 3 * K + 1;
   if (int r = pull_clock(h)) return r;
   const long long m = h->clock.step - step0;
   *taken = m;
@@ -1306,6 +1317,7 @@ static int fused_run(bx_handle* h, double endtime, int64_t nsteps, int64_t* take
     h->p_saved = false;
     h->last_path = 1;
   }
+  if (!h->clock.flags && !h->clock.tripped) return BX_OK;
   h->clock.flags = 0;
   h->clock.tripped = 0;
   h->clock.active = 0;

@@ -4,8 +4,8 @@
 // one table of per-box geometry and clocks, and one tile list that covers every
 // box: TX x TY interior column tiles (z split into chunks of at most 32 planes for
 // large boxes), ordered by decreasing work so that the block scheduler hands the
-// longest tiles out first.  A step is four launches for the whole ensemble --
-// per-box dt control, stage 0, stage 1, per-box clock advance -- the same stage
+// longest tiles out first.  A step is three launches for the whole ensemble --
+// stage 0, stage 1, and per box the clock advance with the next dt -- the same stage
 // kernels as the single-grid path, so each box evolves bit for bit as it would
 // alone.  A run of n steps is captured once into a CUDA graph and replayed.
 //
@@ -446,7 +446,7 @@ static int enqueue_steps(bx_batch* b, int nsteps) {
   for (int k = 0; k < nsteps; ++k) {
     const int X = c, Y = (c + 1) % 3, Z = (c + 2) % 3;
     b->step_x[k] = X;
-    BCK(launch_dt_batch(b->d_ctrl, b->nbox, b->stream));
+    if (k == 0) BCK(launch_dt_batch(b->d_ctrl, b->nbox, b->stream));
     a.X = b->buf[X];
     a.Y = nullptr;
     a.out = b->buf[Y];
@@ -454,7 +454,8 @@ static int enqueue_steps(bx_batch* b, int nsteps) {
     a.Y = b->buf[Y];
     a.out = b->buf[Z];
     BCK(launch_stage(1, b->pm, b->threed, a, b->ntiles, b->stream, b->shape));
-    BCK(launch_end_batch(b->d_ctrl, b->nbox, b->stream));
+    BCK(k + 1 < nsteps ? launch_next_batch(b->d_ctrl, b->nbox, b->stream)
+                       : launch_end_batch(b->d_ctrl, b->nbox, b->stream));
     c = Z;
   }
   return BX_OK;
@@ -512,7 +513,7 @@ int bx_batch_run(bx_batch* b, int64_t nsteps, double endtime, int32_t use_graph)
   float ms = 0.f;
   BCK(cudaEventElapsedTime(&ms, b->ev0, b->ev1));
   b->last_ms = ms;
-  b->last_launches = b->persistent ? 3 : 4ll * ns;
+  b->last_launches = b->persistent ? 3 : 3ll * ns + 1;
   if (b->persistent) {
     int st = 0;
     BCK(cudaMemcpy(&st, b->d_pstatus, sizeof(int), cudaMemcpyDeviceToHost));
@@ -561,7 +562,7 @@ int bx_batch_run(bx_batch* b, int64_t nsteps, double endtime, int32_t use_graph)
 // depths, and 64, 32, 16 and 8 planes) runs `reps` trial steps from the boxes'
 // current states -- a step reads the input plane set and writes the other two,
 // and the clocks are put back after every trial, so the ensemble is left as it
-// was -- with four launches per step; at the fastest shape and depth the
+// was -- with three launches per step; at the fastest shape and depth the
 // persistent launch is timed the same way, and the faster of the two launch
 // forms stays.  The halo is the stencil's two cells (a deeper halo would fuse
 // the two stages at the cost of recomputing stage 0 on a two-cell ring around

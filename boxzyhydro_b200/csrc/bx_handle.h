@@ -48,6 +48,7 @@ struct bx_handle {
   bool gforce_set = false;
   uint32_t status = 0;
   int last_path = 0;
+  cudaEvent_t ev_copied = nullptr;  // bx_set_phi: the host's array has been read
   // profiling: CUDA events around the stage launches, accumulated per step
   bool prof = false;
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};

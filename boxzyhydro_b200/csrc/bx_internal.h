@@ -194,6 +194,12 @@ int stage_blocks_per_sm(int stage, int pm, bool threed, int shape = 0);
 cudaError_t launch_stage(int stage, int pm, bool threed, const StageArgs& a, int ntiles,
                          cudaStream_t s, int shape = 0);
 cudaError_t launch_dt(Ctrl* ctrl, int nbox, cudaStream_t s);
+// one box: launch_dt with the step's dt into *record; launch_end and, if record is not
+// null, the next step's launch_begin_run
+cudaError_t launch_begin_run(Ctrl* ctrl, double* record, cudaStream_t s);
+cudaError_t launch_next_run(Ctrl* ctrl, double* record, cudaStream_t s);
+// launch_end_batch, then the next step's launch_dt_batch
+cudaError_t launch_next_batch(Ctrl* ctrl, int nbox, cudaStream_t s);
 cudaError_t launch_end(Ctrl* ctrl, int nbox, cudaStream_t s);
 
 // phase kernels (one reference subroutine each, full arrays)

@@ -169,16 +169,60 @@ __device__ __forceinline__ void load_vec(const double* U, long long PS, const Pl
   if (p.fz) u3 = -u3;
 }
 
-// source(0) with gravity on conserved values c (source.f90:161-182 with dt/2):
-// the velocity array it reads is m/rho before the kick (the last velocity() ran
-// on these momenta); returns that velocity in (v1, v2, v3) for state()
-__device__ __forceinline__ void gravity_source0(Cons& c, double g1, double g2, double g3,
-                                                double dth, double small_eps, double& v1,
-                                                double& v2, double& v3) {
-  v1 = c.m1 / c.d;
-  v2 = c.m2 / c.d;
-  v3 = c.m3 / c.d;
-  source_gravity(c.d, c.m1, c.m2, c.m3, c.E, g1, g2, g3, v1, v2, v3, dth, small_eps);
+// The quotients of one cell's numerators by its density d.  FAST: through one
+// correctly rounded reciprocal, exact while ok stays true (the window check of
+// every numerator, looked at once, by the caller); otherwise IEEE, out of line.
+template <bool FAST>
+struct CellDiv {
+  double d, r;
+  bool ok;
+  __device__ __forceinline__ explicit CellDiv(double den) : d(den) {
+    ok = !FAST || den_fast_ok(den);
+    r = FAST ? rcp_fast(den) : 0.0;
+  }
+  __device__ __forceinline__ double operator()(double a) {
+    if (!FAST) return div_ieee(a, d);
+    ok = ok && quot_fast_ok(a);
+    return quot_fast(a, d, r);
+  }
+  __device__ __forceinline__ double root(double a) {  // sqrt(a/d)
+    if (!FAST) return sound_ieee(a, d);
+    ok = ok && rad_fast_ok(a);
+    return sqrt_fast(quot_fast(a, d, r));
+  }
+};
+
+// source() with a force on a cell (source.f90:161-182), the velocity (u1, u2, u3)
+// being the array's from before it
+template <class Div>
+__device__ __forceinline__ void force_source(Div& qd, double& m1, double& m2, double& m3, double& E,
+                                             double g1, double g2, double g3, double u1, double u2,
+                                             double u3, double dt, double small_eps) {
+  const double d = qd.d;
+  m2 = m2 + (d * (g2)) * dt;
+  m1 = m1 + (d * (g1)) * dt;
+  m3 = m3 + ((g3) * d) * dt;
+  const double ek = qd(kHalf * (m1 * m1 + m2 * m2 + m3 * m3));
+  E = at_least(E - ek + dt * d * (((u1) * (g1) + (u2) * (g2) + (u3) * (g3))), small_eps) + ek;
+}
+
+// The sources before flux(0) of a step with a force: the nsrc-1 force-free ones
+// still pending, then source(0) with the force (dt/2).  The velocity array it
+// reads is m/rho before the kick (the last velocity() ran on these momenta), which
+// is also state()'s: returned in (v1, v2, v3).
+template <class Div>
+__device__ __forceinline__ void force_source0(Div& qd, Cons& c, double g1, double g2, double g3,
+                                              double dth, int nsrc, double small_eps, double& v1,
+                                              double& v2, double& v3) {
+  if (nsrc > 1) {
+    const double ek = qd(kHalf * (c.m1 * c.m1 + c.m2 * c.m2 + c.m3 * c.m3));
+#pragma unroll 1
+    for (int k = 1; k < nsrc; ++k) c.E = at_least(c.E - ek, small_eps) + ek;
+  }
+  v1 = qd(c.m1);
+  v2 = qd(c.m2);
+  v3 = qd(c.m3);
+  force_source(qd, c.m1, c.m2, c.m3, c.E, g1, g2, g3, v1, v2, v3, dth, small_eps);
 }
 
 __device__ __forceinline__ void apply_sources(Cons& c, int nsrc, double small_eps) {
@@ -282,6 +326,24 @@ __device__ __forceinline__ Prim prim_ieee(double small_eps, double gm1, double g
   return q;
 }
 
+// stage 0 with the acceleration (g1, g2, g3); false: recompute with FAST = false
+template <bool FAST>
+__device__ __forceinline__ bool prim_force(const Geom& g, Cons c, double g1, double g2, double g3,
+                                           int nsrc, double dth, bool need_c, Prim& q) {
+  CellDiv<FAST> qd(c.d);
+  double v1, v2, v3;
+  force_source0(qd, c, g1, g2, g3, dth, nsrc, g.small_eps, v1, v2, v3);
+  q.d = c.d;
+  q.u1 = qd(c.m1);
+  q.u2 = qd(c.m2);
+  q.u3 = qd(c.m3);
+  q.e = recon_eps(q.d, c.E, q.u1, q.u2, q.u3, g.small_eps);
+  q.p = eos_pressure(q.d, c.E, v1, v2, v3, g.gm1, g.small_eps);
+  // the sound speed enters only the lambdas of cells whose face states are built
+  q.c = need_c ? qd.root(q.p * g.gam) : 0.0;
+  return qd.ok;
+}
+
 template <int STAGE, bool GRAV = false, bool TAB = false>
 __device__ __forceinline__ Prim prim_of(const Geom& g, Raw r, int nsrc, double dth,
                                         bool need_c = true, int rs = 0,
@@ -289,19 +351,8 @@ __device__ __forceinline__ Prim prim_of(const Geom& g, Raw r, int nsrc, double d
   Prim q;
   q.g = g.gam;
   if (STAGE == 0 && GRAV) {
-    const SharedDiv qd(r.c.d);
-    Cons c = r.c;
-    double v1, v2, v3;
-    apply_sources(c, nsrc - 1, g.small_eps);
-    gravity_source0(c, r.v1, r.v2, r.v3, dth, g.small_eps, v1, v2, v3);
-    q.d = c.d;
-    q.u1 = qd(c.m1);
-    q.u2 = qd(c.m2);
-    q.u3 = qd(c.m3);
-    q.e = recon_eps(q.d, c.E, q.u1, q.u2, q.u3, g.small_eps);
-    q.p = eos_pressure(q.d, c.E, v1, v2, v3, g.gm1, g.small_eps);
-    // the sound speed enters only the lambdas of cells whose face states are built
-    q.c = need_c ? sqrt(qd(q.p * g.gam)) : 0.0;
+    if (!prim_force<true>(g, r.c, r.v1, r.v2, r.v3, nsrc, dth, need_c, q))
+      prim_force<false>(g, r.c, r.v1, r.v2, r.v3, nsrc, dth, need_c, q);
   } else if (!prim_fast<STAGE>(g, r.c, r.v1, r.v2, r.v3, nsrc, need_c && !TAB, q, rs)) {
     q = prim_ieee<STAGE>(g.small_eps, g.gm1, g.gam, r.c, r.v1, r.v2, r.v3, nsrc,
                          need_c && !TAB, rs);
@@ -485,6 +536,31 @@ __device__ __forceinline__ void epi_ieee(const Geom& g, const double n[5], doubl
   r0 = courant_rate<POW2>(n[0], pA, g.gam, u1, u2, u3, g.dx, g.dy, g.dz, g.idx, g.idy, g.idz);
 }
 
+// The same end of stage 1 with a force: the velocity after flux(1), the cell k
+// after source(1) with the force, its velocity w and the next step's Courant rate
+template <bool FAST, bool POW2>
+__device__ __forceinline__ bool epi_force(const Geom& g, const double n[5], double g1, double g2,
+                                          double g3, double dth, double& u1, double& u2, double& u3,
+                                          double k[5], double w[3], double& r0) {
+  CellDiv<FAST> qd(n[0]);
+#pragma unroll
+  for (int q = 0; q < 5; ++q) k[q] = n[q];
+  u1 = qd(k[1]);
+  u2 = qd(k[2]);
+  u3 = qd(k[3]);
+  force_source(qd, k[1], k[2], k[3], k[4], g1, g2, g3, u1, u2, u3, dth, g.small_eps);
+#pragma unroll
+  for (int q = 0; q < 3; ++q) w[q] = qd(k[1 + q]);
+  const double pA = eos_pressure(k[0], k[4], w[0], w[1], w[2], g.gm1, g.small_eps);
+  const double sound = qd.root(g.gam * pA);
+  if (POW2)
+    r0 = (sound + fabs(w[0])) * g.idx + (sound + fabs(w[1])) * g.idy + (sound + fabs(w[2])) * g.idz;
+  else
+    r0 = cdiv(sound + fabs(w[0]), g.dx, g.idx) + cdiv(sound + fabs(w[1]), g.dy, g.idy) +
+         cdiv(sound + fabs(w[2]), g.dz, g.idz);
+  return qd.ok;
+}
+
 // The same end of stage 1 with the tabulated EOS: the next step's state()
 // takes p and gamma from the tables (state.f90:60-79) with the velocity after
 // source(1), m/rho of the new cell, and courant.f90:20-21 uses that gamma.
@@ -503,6 +579,67 @@ __device__ __forceinline__ void epi_tab(const Geom& g, const EosDev& eos, const 
   r0 = courant_rate_q<POW2>(qn, p, gam, u1, u2, u3, g.dx, g.dy, g.dz, g.idx, g.idy, g.idz);
 }
 
+// A batched box's clock at the start of a step (dt control of main.f90:266-281
+// and 342, with the clock saved for a trip) and at its end (main.f90:471,544-545,
+// or the trip of a box whose step raised a guard: its planes then keep the
+// step's input and its clock is put back)
+__device__ __forceinline__ void box_begin_step(Ctrl& c) {
+  c.run_step += 1;
+  if (c.tripped || !(c.time < c.endtime) || c.step >= 1000000 || c.step >= c.max_step) {
+    c.active = 0;
+    return;
+  }
+  c.time0 = c.time;
+  c.dtold0 = c.dtold;
+  c.step0 = c.step;
+  c.rate_bits0 = c.rate_bits;
+  c.step = c.step + 1;
+  const double rate = __longlong_as_double((long long)c.rate_bits);
+  c.rate = rate;
+  c.rate_bits = 0ull;
+  double dt = c.cfl / rate;
+  dt = dt * 1.0;
+  if (c.step > 1 && c.dtold > 0.0) dt = fmin(dt, c.dtold * 1.1);
+  c.dtold = dt;
+  if (dt + c.time > c.endtime) dt = c.endtime - c.time;
+  dt = dt * kHalf;
+  dt = dt * 2.0;
+  c.dt = dt;
+  c.active = 1;
+}
+__device__ __forceinline__ void box_end_step(Ctrl& c) {
+  if (!c.active) return;
+  if (c.flags & (kFlagVlimit | kFlagLowRho | kFlagNonFinite)) {
+    c.tripped = 1;
+    c.trip_step = c.run_step - 1;
+    c.time = c.time0;
+    c.dtold = c.dtold0;
+    c.step = c.step0;
+    c.rate_bits = c.rate_bits0;
+    c.active = 0;
+    return;
+  }
+  double dt = kHalf * c.dt;
+  dt = dt * 2.0;
+  c.time = c.time + dt;
+  c.nsrc = 2;
+}
+static_assert(sizeof(Ctrl) % 8 == 0, "Ctrl moves as 8-byte words");
+// a box's control block through L2 (other blocks of the launch write it)
+__device__ __forceinline__ Ctrl ctrl_load_cg(const Ctrl* p) {
+  Ctrl c;
+  const unsigned long long* s = reinterpret_cast<const unsigned long long*>(p);
+  unsigned long long* d = reinterpret_cast<unsigned long long*>(&c);
+#pragma unroll
+  for (int k = 0; k < (int)(sizeof(Ctrl) / 8); ++k) d[k] = __ldcg(s + k);
+  return c;
+}
+__device__ __forceinline__ void ctrl_store_cg(Ctrl* p, const Ctrl& c) {
+  unsigned long long* d = reinterpret_cast<unsigned long long*>(p);
+  const unsigned long long* s = reinterpret_cast<const unsigned long long*>(&c);
+#pragma unroll
+  for (int k = 0; k < (int)(sizeof(Ctrl) / 8); ++k) __stcg(d + k, s[k]);
+}
 // ------------------------------------------------------------------ stage kernel
 // One tile of one stage: TX x TY columns marched along z.  Per plane:
 //  A  primitives of the tile's cells and its two-cell x/y halo to shared memory
@@ -598,7 +735,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
 
   // the halo cell of this thread (those without a column first), if any
   static_assert(4 * (TX + TY) <= NT, "one halo cell per thread and plane at most");
-  long long hpc = 0;
+  long long hpc = 0;  // its column
   int hc = -1;  // its place in SP
   {
     const int i = (tid + NT - NOWN) % NT;
@@ -812,9 +949,15 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
           ft[q] = POW2 ? -sum * dt * g.ivol : cdiv(-sum * dt, g.vol, g.ivol);
         }
         if (GRAV) {
+          const Cons cx = c0;
           double v1, v2, v3;
-          apply_sources(c0, nsrc - 1, g.small_eps);
-          gravity_source0(c0, go1, go2, go3, dth, g.small_eps, v1, v2, v3);
+          CellDiv<true> qf(cx.d);
+          force_source0(qf, c0, go1, go2, go3, dth, nsrc, g.small_eps, v1, v2, v3);
+          if (!qf.ok) {
+            CellDiv<false> qs(cx.d);
+            c0 = cx;
+            force_source0(qs, c0, go1, go2, go3, dth, nsrc, g.small_eps, v1, v2, v3);
+          }
         } else {
           const SharedDiv q0(c0.d);
 #pragma unroll 1
@@ -857,10 +1000,22 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
           // reciprocal and one window check for all of them (epi_fast)
           double u1, u2, u3, r0 = 0.0;
           if (GRAV) {
-            const SharedDiv qn(n[0]);
-            u1 = qn(n[1]);
-            u2 = qn(n[2]);
-            u3 = qn(n[3]);
+            double k[5], w[3];
+            if (!epi_force<true, POW2>(g, n, go1, go2, go3, dth, u1, u2, u3, k, w, r0))
+              epi_force<false, POW2>(g, n, go1, go2, go3, dth, u1, u2, u3, k, w, r0);
+            // source(1) with the force (main.f90:471): the planes take its result,
+            // the velocity it read goes to UC for state() at the step's end
+            // (main.f90:513-514), and the Courant rate of the next step is taken
+            // with the velocity after it (main.f90:515)
+            a.UC[o] = u1;
+            a.UC[PS + o] = u2;
+            a.UC[2 * PS + o] = u3;
+            if (fabs(w[0]) > g.vlimit || fabs(w[1]) > g.vlimit || fabs(w[2]) > g.vlimit)
+              flags |= kFlagVlimit;
+            if (!(isfinite(k[1]) && isfinite(k[2]) && isfinite(k[3]) && isfinite(k[4])))
+              flags |= kFlagNonFinite;
+#pragma unroll
+            for (int q = 1; q < 5; ++q) n[q] = k[q];
           } else if (TAB) {
             epi_tab<POW2>(g, a.eos, n, u1, u2, u3, r0);
           } else if (!epi_fast<POW2>(g, n, u1, u2, u3, r0)) {
@@ -869,30 +1024,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
           if (n[0] < kLowRho) flags |= kFlagLowRho;
           if (fabs(u1) > g.vlimit || fabs(u2) > g.vlimit || fabs(u3) > g.vlimit)
             flags |= kFlagVlimit;
-          if (GRAV) {
-            // source(1) with the force (main.f90:471): the planes take its result,
-            // the velocity it read goes to UC for state() at the step's end
-            // (main.f90:513-514), and the Courant rate of the next step is taken
-            // with the velocity after it (main.f90:515)
-            a.UC[o] = u1;
-            a.UC[PS + o] = u2;
-            a.UC[2 * PS + o] = u3;
-            source_gravity(n[0], n[1], n[2], n[3], n[4], go1, go2, go3, u1, u2, u3, dth,
-                           g.small_eps);
-            const double w1 = n[1] / n[0], w2 = n[2] / n[0], w3 = n[3] / n[0];
-            if (fabs(w1) > g.vlimit || fabs(w2) > g.vlimit || fabs(w3) > g.vlimit)
-              flags |= kFlagVlimit;
-            if (!(isfinite(n[1]) && isfinite(n[2]) && isfinite(n[3]) && isfinite(n[4])))
-              flags |= kFlagNonFinite;
-            const double pA = eos_pressure(n[0], n[4], w1, w2, w3, g.gm1, g.small_eps);
-            const double r0 = courant_rate<POW2>(n[0], pA, g.gam, w1, w2, w3, g.dx, g.dy, g.dz,
-                                                 g.idx, g.idy, g.idz);
-            rate = at_least(r0, rate);
-            if (!(r0 >= 0.0)) flags |= kFlagNonFinite;
-          } else {
-            rate = at_least(r0, rate);
-            if (!(r0 >= 0.0)) flags |= kFlagNonFinite;
-          }
+          rate = at_least(r0, rate);
+          if (!(r0 >= 0.0)) flags |= kFlagNonFinite;
         }
 #pragma unroll
         for (int q = 0; q < 5; ++q) a.out[q * PS + o] = n[q];
@@ -959,51 +1092,6 @@ __global__ void __launch_bounds__(ShapeSel<SH>::type::NT, 2) k_stage(StageArgs a
   stage_tile<S, STAGE, PM == 1, THREED, GRAV>(a, t, sg, C, dt, nsrc, sm, red_rate, red_flags);
 }
 
-// A batched box's clock at the start of a step (dt control of main.f90:266-281
-// and 342, with the clock saved for a trip) and at its end (main.f90:471,544-545,
-// or the trip of a box whose step raised a guard: its planes then keep the
-// step's input and its clock is put back)
-__device__ __forceinline__ void box_begin_step(Ctrl& c) {
-  c.run_step += 1;
-  if (c.tripped || !(c.time < c.endtime) || c.step >= 1000000 || c.step >= c.max_step) {
-    c.active = 0;
-    return;
-  }
-  c.time0 = c.time;
-  c.dtold0 = c.dtold;
-  c.step0 = c.step;
-  c.rate_bits0 = c.rate_bits;
-  c.step = c.step + 1;
-  const double rate = __longlong_as_double((long long)c.rate_bits);
-  c.rate = rate;
-  c.rate_bits = 0ull;
-  double dt = c.cfl / rate;
-  dt = dt * 1.0;
-  if (c.step > 1 && c.dtold > 0.0) dt = fmin(dt, c.dtold * 1.1);
-  c.dtold = dt;
-  if (dt + c.time > c.endtime) dt = c.endtime - c.time;
-  dt = dt * kHalf;
-  dt = dt * 2.0;
-  c.dt = dt;
-  c.active = 1;
-}
-__device__ __forceinline__ void box_end_step(Ctrl& c) {
-  if (!c.active) return;
-  if (c.flags & (kFlagVlimit | kFlagLowRho | kFlagNonFinite)) {
-    c.tripped = 1;
-    c.trip_step = c.run_step - 1;
-    c.time = c.time0;
-    c.dtold = c.dtold0;
-    c.step = c.step0;
-    c.rate_bits = c.rate_bits0;
-    c.active = 0;
-    return;
-  }
-  double dt = kHalf * c.dt;
-  dt = dt * 2.0;
-  c.time = c.time + dt;
-  c.nsrc = 2;
-}
 namespace {
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   unsigned v;
@@ -1017,22 +1105,6 @@ __device__ bool wait_at_least(const unsigned* p, unsigned target, long long limi
     __nanosleep(100);
   }
   return false;
-}
-static_assert(sizeof(Ctrl) % 8 == 0, "Ctrl moves as 8-byte words");
-// a box's control block through L2 (other blocks of the launch write it)
-__device__ __forceinline__ Ctrl ctrl_load_cg(const Ctrl* p) {
-  Ctrl c;
-  const unsigned long long* s = reinterpret_cast<const unsigned long long*>(p);
-  unsigned long long* d = reinterpret_cast<unsigned long long*>(&c);
-#pragma unroll
-  for (int k = 0; k < (int)(sizeof(Ctrl) / 8); ++k) d[k] = __ldcg(s + k);
-  return c;
-}
-__device__ __forceinline__ void ctrl_store_cg(Ctrl* p, const Ctrl& c) {
-  unsigned long long* d = reinterpret_cast<unsigned long long*>(p);
-  const unsigned long long* s = reinterpret_cast<const unsigned long long*>(&c);
-#pragma unroll
-  for (int k = 0; k < (int)(sizeof(Ctrl) / 8); ++k) __stcg(d + k, s[k]);
 }
 }  // namespace
 
@@ -1248,11 +1320,8 @@ size_t stage_smem_bytes(int shape) {
 }
 
 // ------------------------------------------------------------------ clock kernels
-// dt control of main.f90:266-281 and 342, per box
-__global__ void k_dt(Ctrl* ctrl, int n) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
-  Ctrl& c = ctrl[b];
+// dt control of main.f90:266-281 and 342
+__device__ __forceinline__ void clock_begin(Ctrl& c) {
   if (!(c.time < c.endtime) || c.step >= 1000000 || c.step >= c.max_step) {
     c.active = 0;
     return;
@@ -1271,16 +1340,41 @@ __global__ void k_dt(Ctrl* ctrl, int n) {
   c.dt = dt;
   c.active = 1;
 }
-
 // main.f90:471,544-545
-__global__ void k_end(Ctrl* ctrl, int n) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
-  Ctrl& c = ctrl[b];
+__device__ __forceinline__ void clock_end(Ctrl& c) {
   if (!c.active) return;
   double dt = kHalf * c.dt;
   dt = dt * 2.0;
   c.time = c.time + dt;
+}
+__global__ void k_dt(Ctrl* ctrl, int n) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < n) clock_begin(ctrl[b]);
+}
+__global__ void k_end(Ctrl* ctrl, int n) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < n) clock_end(ctrl[b]);
+}
+
+// Between two steps of a run one launch ends the one and begins the next (a small
+// grid's step is launches of a few microseconds each: 512-cell tube 17.0 us a step
+// with four of them and two copies of the control block around a chunk, 15.3 with
+// three and none).  record: receives the step's dt.
+__global__ void k_begin_run(Ctrl* c, double* record) {
+  clock_begin(*c);
+  *record = c->dt;
+}
+__global__ void k_next_run(Ctrl* c, double* record) {
+  clock_end(*c);
+  if (!record) return;
+  clock_begin(*c);
+  *record = c->dt;
+}
+__global__ void k_next_batch(Ctrl* ctrl, int n) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= n) return;
+  box_end_step(ctrl[b]);
+  box_begin_step(ctrl[b]);
 }
 
 // batched boxes: as k_dt/k_end, plus the saved clock and the trip of a box
@@ -1306,6 +1400,18 @@ cudaError_t launch_end_batch(Ctrl* ctrl, int nbox, cudaStream_t s) {
 
 cudaError_t launch_dt(Ctrl* ctrl, int nbox, cudaStream_t s) {
   k_dt<<<(nbox + 127) / 128, 128, 0, s>>>(ctrl, nbox);
+  return cudaGetLastError();
+}
+cudaError_t launch_begin_run(Ctrl* ctrl, double* record, cudaStream_t s) {
+  k_begin_run<<<1, 1, 0, s>>>(ctrl, record);
+  return cudaGetLastError();
+}
+cudaError_t launch_next_run(Ctrl* ctrl, double* record, cudaStream_t s) {
+  k_next_run<<<1, 1, 0, s>>>(ctrl, record);
+  return cudaGetLastError();
+}
+cudaError_t launch_next_batch(Ctrl* ctrl, int nbox, cudaStream_t s) {
+  k_next_batch<<<(nbox + 127) / 128, 128, 0, s>>>(ctrl, nbox);
   return cudaGetLastError();
 }
 cudaError_t launch_end(Ctrl* ctrl, int nbox, cudaStream_t s) {

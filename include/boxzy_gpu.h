@@ -244,7 +244,7 @@ int bx_ghost_plan(const bx_params *params, int64_t *nghost, int32_t *dst, int32_
 
 /* ---- Batched ensembles.  No counterpart in the reference, which advances one grid
  * per process.  Many independent grids ("boxes", each with its own size, gamma, cfl,
- * dt and clock) advance together: one tile list spans all boxes, a step is four
+ * dt and clock) advance together: one tile list spans all boxes, a step is three
  * launches for the whole ensemble, and a run of n steps is replayed as one CUDA
  * graph.  Each box evolves bit for bit as it would under bx_step on its own.  Boxes
  * must be fused-eligible (bx_ghost_plan fused_ok) and all 3-D (nz>=6) or all 2-D;
@@ -261,7 +261,7 @@ int bx_batch_set_clock(bx_batch *b, int32_t box, double time, double dtold, int6
 int bx_batch_get_clock(bx_batch *b, int32_t box, double *time, double *dt, double *dtold,
                        int64_t *step);
 /* nsteps iterations of every box's main loop (boxes at endtime stop).  use_graph != 0:
- * the run is captured once into a CUDA graph and replayed.  The launches are four per
+ * the run is captured once into a CUDA graph and replayed.  The launches are three per
  * step (dt, stage 0, stage 1, clock), or, in persistent mode (bx_batch_set_persistent,
  * or chosen by bx_batch_autotune), one launch for the whole run after the first
  * step's dt: its blocks take (step, stage, tile) items from a queue in step order and
