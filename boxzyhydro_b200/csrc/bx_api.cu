@@ -193,6 +193,9 @@ static int create_handle(const bx_params* params, bx_handle** out, bool lean) {
   h->ntiles = (int)tiles.size();
   CKC(dalloc((void**)&h->d_tiles, tiles.size() * sizeof(Tile)));
   CKC(cudaMemcpy(h->d_tiles, tiles.data(), tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice));
+  h->pa.geom = h->d_geom;
+  h->pa.tiles = h->d_tiles;
+  h->pa.ntiles = h->ntiles;
   CKC(dalloc((void**)&h->d_ctrl, sizeof(Ctrl)));
   CKC(cudaMallocHost((void**)&h->h_ctrl, sizeof(Ctrl)));
   std::memset(&h->clock, 0, sizeof(Ctrl));
@@ -275,7 +278,8 @@ static int push_clock(bx_handle* h) {
 
 static int ensure_states(bx_handle* h) {
   if (!h->pa.states)
-    CK(dalloc((void**)&h->pa.states, (h->g.ang ? 54 : 57) * h->g.ng * sizeof(double)));
+    CK(dalloc((void**)&h->pa.states,
+              (h->g.ang ? 54 : h->g.tab ? 57 : 5) * h->g.ng * sizeof(double)));
   return BX_OK;
 }
 
@@ -665,8 +669,10 @@ int bx_device_cons(bx_handle* h, double** cons_soa, int64_t* ngrid) {
 }
 
 // ---- whole steps
-static int ghost1(bx_handle* h) {
-  CK(phase_ghost(h->nghost, h->d_dst, h->d_src1, h->d_sgn1, h->pa, h->g.ng, h->stream));
+// two consecutive ghost fills (main.f90:312,351,374,511 after those of source and
+// flux): the composed plan, every source read before the first of them
+static int ghost2(bx_handle* h) {
+  CK(phase_ghost(h->nghost, h->d_dst, h->d_src2, h->d_sgn2, h->pa, h->g.ng, h->stream));
   return BX_OK;
 }
 
@@ -682,28 +688,19 @@ static int phase_step(bx_handle* h) {
   CK(phase_courant(g, a, c, s));
   CK(launch_dt(c, 1, s));
   CK(phase_source(g, a, c, 0.5, s));   // source(time,0) with dt/2
-  if (int r = ghost1(h)) return r;
-  if (int r = ghost1(h)) return r;     // main.f90:312
-  CK(phase_state(g, a, c, s));
-  CK(phase_velocity(g, a, c, s));
-  CK(phase_copy_old(g, a, s));
-  CK(phase_flux(g, a, c, 0, s));
-  if (int r = ghost1(h)) return r;     // flux.f90:231
-  if (int r = ghost1(h)) return r;     // main.f90:351
-  CK(phase_state(g, a, c, s));
-  CK(phase_velocity(g, a, c, s));
+  if (int r = ghost2(h)) return r;
+  CK(phase_state_velocity(g, a, c, s));
+  CK(phase_flux(g, a, c, 0, s, true));  // main.f90:327-333 first
+  if (int r = ghost2(h)) return r;     // flux.f90:231, main.f90:351
+  CK(phase_state_velocity(g, a, c, s));
   CK(phase_flux(g, a, c, 1, s));
-  if (int r = ghost1(h)) return r;
-  if (int r = ghost1(h)) return r;     // main.f90:374
-  CK(phase_state(g, a, c, s));
-  CK(phase_velocity(g, a, c, s));
+  if (int r = ghost2(h)) return r;
+  CK(phase_state_velocity(g, a, c, s));
   CK(phase_source(g, a, c, 0.5, s));   // source(time+dt,1) with dt/2
-  if (int r = ghost1(h)) return r;
-  if (int r = ghost1(h)) return r;     // main.f90:511
-  CK(phase_state(g, a, c, s));
-  CK(phase_velocity(g, a, c, s));
+  if (int r = ghost2(h)) return r;
+  CK(phase_state_velocity(g, a, c, s));
   CK(launch_end(c, 1, s));
-  h->launches += 46;
+  h->launches += 22 + (g.ang || g.tab ? 3 : 0);
   return BX_OK;
 }
 
@@ -770,8 +767,10 @@ static int phase_path(bx_handle* h, int32_t* ran) {
   h->status |= f;
   h->last_path = 0;
   if (ran) *ran = 1;
-  h->clock.flags = 0;
-  if (int r = push_clock(h)) return r;
+  if (f) {  // (otherwise the device's block is the mirror's already)
+    h->clock.flags = 0;
+    if (int r = push_clock(h)) return r;
+  }
   if (f & kFlagNonFinite) return set_err(h, BX_ERR_STATE, "non-finite state produced by the step");
   if (h->eligible && !(f & (kFlagVlimit | kFlagLowRho))) return enter_fused(h);
   return BX_OK;
@@ -1179,8 +1178,8 @@ int bx_handle_start_from_planes(bx_handle* h, const double* planes) {
   const long long n = h->g.ng;
   cudaStream_t s = h->stream;
   CK(cudaMemcpyAsync(h->pa.cons, planes, 5 * n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  for (int k = 0; k < 4; ++k)
-    if (int r = ghost1(h)) return r;
+  for (int k = 0; k < 2; ++k)
+    if (int r = ghost2(h)) return r;
   CK(prims_from_cons(h->g, h->pa, s));
   h->launches += 5;
   h->mode = 0;

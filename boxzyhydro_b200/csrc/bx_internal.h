@@ -169,6 +169,7 @@ struct StageArgs {
   double* U;         // 3 planes: stage 0 writes m/rho of the step input at its own
                      // cells, stage 1 reads it as the stale velocity of its EOS
   const double* G;   // 3 planes of the gravitational acceleration, or null (no force)
+  const double* P;   // the reference's pressure array (the per-phase flux only)
   double* UC;        // with G: stage 1 writes the velocity after flux(1) of its
                      // own cells (the velocity state() reads at the step's end)
   Ctrl* ctrl;        // per box control blocks
@@ -210,21 +211,28 @@ struct PhaseArrays {
   double* p;        // ng
   double* adindx;   // ng
   double* gforce;   // 3*ng or null (zero force)
-  double* states;   // flux scratch: 42*ng face states, then 15*ng face fluxes
-                    // (fixed frame); 54*ng face states with fluxangmom
+  double* states;   // flux scratch: 5*ng, the interior cells' result (fixed gamma);
+                    // 42*ng face states, then 15*ng face fluxes (tabulated EOS);
+                    // 54*ng face states (fluxangmom)
   double* gtmp;     // 5*nghost scratch for the ghost fill
   double* muc;      // ng (H2STAT >= 0: muc_array of state(); else null)
   EosDev eos;       // valid when muc is set
+  const Geom* geom; // the grid on the device, and its stage-kernel tiles (the flux
+  const Tile* tiles;// with fixed gamma)
+  int ntiles;
 };
 
 cudaError_t phase_state(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream_t s);
 cudaError_t phase_velocity(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream_t s);
+cudaError_t phase_state_velocity(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream_t s);
 cudaError_t phase_courant(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream_t s);
 cudaError_t phase_source(const Geom& g, PhaseArrays& a, Ctrl* ctrl, double mult, cudaStream_t s);
 cudaError_t phase_calc_gforce(const Geom& g, const double* phi, double* gforce, cudaStream_t s);
 cudaError_t phase_ghost(int nghost, const int32_t* dst, const int32_t* src, const uint8_t* sgn,
                         PhaseArrays& a, long long ng, cudaStream_t s);
-cudaError_t phase_flux(const Geom& g, PhaseArrays& a, Ctrl* ctrl, int avg, cudaStream_t s);
+// save_old: phase_copy_old first
+cudaError_t phase_flux(const Geom& g, PhaseArrays& a, Ctrl* ctrl, int avg, cudaStream_t s,
+                       bool save_old = false);
 cudaError_t phase_courant_finish(Ctrl* ctrl, cudaStream_t s);
 // avisc.f90:13-23 into qq (3 planes of ng) from the velocity array u
 cudaError_t phase_avisc(const Geom& g, const double* u, const double avmag[3], double* qq,

@@ -244,9 +244,10 @@ __device__ __forceinline__ void apply_sources(Cons& c, int nsrc, double small_ep
 // The values a cell's primitives are computed from: its conserved variables
 // (X in stage 0, Y in stage 1) and, in stage 1, the stage-0 velocity U, or,
 // in stage 0 with a force, the acceleration G.
+// (PH, the reference's arrays: the cell's u in v and its p)
 struct Raw {
   Cons c;
-  double v1, v2, v3;
+  double v1, v2, v3, p;
 };
 
 // STAGE 0 or 1: the stage is known at compile time; STAGE 2: it is the runtime
@@ -680,7 +681,10 @@ __device__ __forceinline__ void ctrl_store_cg(Ctrl* p, const Ctrl& c) {
 // persistent batched kernel).
 enum : unsigned { kItemY = 1u << 12, kItemGhost = 1u << 13, kItemIn = 1u << 14 };
 
-template <class S, int STAGE, bool POW2, bool THREED, bool GRAV, bool CG = false>
+// PH: the flux of the per-phase path (flux.f90:6-230) on the reference's arrays:
+// u and p are read, not derived, ghost cells are cells like any other, and nothing of
+// the sources, guards or the next step's rate is done here (phase_flux).
+template <class S, int STAGE, bool POW2, bool THREED, bool GRAV, bool CG = false, bool PH = false>
 __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, const Geom& g,
                                            Ctrl* C, double dt, int nsrc, double* sm,
                                            double* red_rate, unsigned* red_flags, int rs = 0) {
@@ -753,7 +757,9 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
       in = j < 4 && cx < w;
     }
     if (in) {
-      const Place p = place_of(g, bx0 + cx, by0 + cy, g.az0);
+      Place p{g.base + bx0 + cx + (long long)(by0 + cy) * g.sy + (long long)g.az0 * g.sz,
+              false, false, false};
+      if (!PH) p = place_of(g, bx0 + cx, by0 + cy, g.az0);
       hpc = p.c - (long long)g.az0 * g.sz;
       // (a halo cell of the x/y halo is beyond one wall at most)
       hc = ((cy + 2) * PW + cx + 2) | (p.fx ? 1 << 12 : 0) | (p.fy ? 1 << 13 : 0);
@@ -763,11 +769,33 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
   auto zs = [&](int k) -> double& { return ZS[k * NOWN + tid]; };
   auto own_place = [&](int z) {
     Place p{0, false, false, false};
-    const int zz = THREED ? remap_axis(z, g.az0, g.az1, g.wall[4], g.wall[5], p.fz) : z;
+    const int zz = THREED && !PH ? remap_axis(z, g.az0, g.az1, g.wall[4], g.wall[5], p.fz) : z;
     p.c = co + (long long)zz * g.sz;
     return p;
   };
+  auto load_at = [&](const Place& p) {
+    if constexpr (PH) {
+      Raw r;
+      r.c = load_cons(is0 ? a.X : a.Y, PS, p);
+      load_vec(a.U, PS, p, r.v1, r.v2, r.v3);
+      r.p = ldg(a.P + p.c);
+      return r;
+    } else {
+      return load_raw<STAGE, GRAV, CG>(a, p, rs);
+    }
+  };
   auto prim_at = [&](const Raw& r, int x, int y) {
+    if constexpr (PH) {
+      Prim q;
+      q.d = r.c.d;
+      q.u1 = r.v1;
+      q.u2 = r.v2;
+      q.u3 = r.v3;
+      q.p = r.p;
+      q.e = recon_eps(q.d, r.c.E, q.u1, q.u2, q.u3, g.small_eps);
+      q.c = sound_of(q.p * g.gam, q.d);
+      return q;
+    }
     Prim q = prim_of<STAGE, GRAV, TAB>(g, r, nsrc, dth, true, rs, &a.eos);
     // with flux_ang the momenta reconstructed are the transformed ones (the
     // sources leave the momenta alone)
@@ -778,8 +806,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
   // z pipeline of the own column (3-D grids): primitives of planes z and z+1
   Prim Pk, Pk1;
   if (THREED && own) {
-    const Raw r0 = load_raw<STAGE, GRAV, CG>(a, own_place(z0 - 2), rs);
-    const Raw r1 = load_raw<STAGE, GRAV, CG>(a, own_place(z0 - 1), rs);
+    const Raw r0 = load_at(own_place(z0 - 2));
+    const Raw r1 = load_at(own_place(z0 - 1));
     Pk = prim_at(r0, gx, gy);
     Pk1 = prim_at(r1, gx, gy);
   }
@@ -793,7 +821,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
     {
       Raw ro, rh;
       const bool halo = plane && hc >= 0;
-      if (own) ro = load_raw<STAGE, GRAV, CG>(a, own_place(THREED ? z + 2 : z), rs);
+      if (own) ro = load_at(own_place(THREED ? z + 2 : z));
       if (own) {
         // towards L2: the step input that stage 1's update reads at the end of
         // this plane, and the own column's loads of the next plane
@@ -812,10 +840,10 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
         if (plane) {
           put_prim<NP, NPF>(SP, sc, Pk);
           // the guards look at every interior cell where it is an own cell
-          if (Pk.d < kLowRho) flags |= kFlagLowRho;
-          if (fabs(Pk.u1) > g.vlimit || fabs(Pk.u2) > g.vlimit || fabs(Pk.u3) > g.vlimit)
+          if (!PH && Pk.d < kLowRho) flags |= kFlagLowRho;
+          if (!PH && (fabs(Pk.u1) > g.vlimit || fabs(Pk.u2) > g.vlimit || fabs(Pk.u3) > g.vlimit))
             flags |= kFlagVlimit;
-          if (is0) {
+          if (is0 && !PH) {
             // sources change only E, so this is m/rho of the step input
             a.U[o] = Pk.u1;
             a.U[PS + o] = Pk.u2;
@@ -825,7 +853,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
       }
       if (halo) {
         const Place p{hpc + (long long)z * g.sz, (hc & (1 << 12)) != 0, (hc & (1 << 13)) != 0, false};
-        rh = load_raw<STAGE, GRAV, CG>(a, p, rs);
+        rh = load_at(p);
 
         const int k = hc & 0xfff, cy = k / PW - 2, cx = k % PW - 2;
         put_prim<NP, NPF>(SP, k, prim_at(rh, bx0 + cx, by0 + cy));
@@ -958,7 +986,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
             c0 = cx;
             force_source0(qs, c0, go1, go2, go3, dth, nsrc, g.small_eps, v1, v2, v3);
           }
-        } else {
+        } else if (!PH) {
           const SharedDiv q0(c0.d);
 #pragma unroll 1
           for (int k = 0; k < nsrc; ++k)
@@ -994,7 +1022,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
         if (!(isfinite(n[0]) && isfinite(n[1]) && isfinite(n[2]) && isfinite(n[3]) &&
               isfinite(n[4])))
           flags |= kFlagNonFinite;
-        if (!is0) {
+        if (!is0 && !PH) {
           // state/velocity after flux(1) and after source(1) (main.f90:372-380,490-515);
           // without a force every division here is by the new density: one
           // reciprocal and one window check for all of them (epi_fast)
@@ -1050,7 +1078,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
       r = fmax(r, red_rate[k]);
     }
     if (f) atomicOr(&C->flags, f);
-    if (!is0) atomicMax(&C->rate_bits, (unsigned long long)__double_as_longlong(r));
+    if (!is0 && !PH) atomicMax(&C->rate_bits, (unsigned long long)__double_as_longlong(r));
   }
 }
 
@@ -1090,6 +1118,21 @@ __global__ void __launch_bounds__(ShapeSel<SH>::type::NT, 2) k_stage(StageArgs a
   const double dt = C->dt;
   const int nsrc = a.nsrc > 0 ? a.nsrc : C->nsrc;
   stage_tile<S, STAGE, PM == 1, THREED, GRAV>(a, t, sg, C, dt, nsrc, sm, red_rate, red_flags);
+}
+
+// flux(avg) of the per-phase path on the reference's arrays (stage_tile, PH): the
+// interior cells' result to a.out
+template <int AVG, int PM, bool THREED>
+__global__ void __launch_bounds__(Shape0::NT, 2) k_phase_tile(StageArgs a) {
+  extern __shared__ double sm[];
+  __shared__ Geom sg;
+  __shared__ double red_rate[Shape0::NT / 32];
+  __shared__ unsigned red_flags[Shape0::NT / 32];
+  const Tile t = a.tiles[blockIdx.x];
+  if (threadIdx.x == 0) sg = *a.geom;
+  __syncthreads();
+  stage_tile<Shape0, AVG, PM == 1, THREED, false, false, true>(a, t, sg, a.ctrl, a.ctrl->dt, 0, sm,
+                                                               red_rate, red_flags);
 }
 
 namespace {
@@ -1431,9 +1474,8 @@ __device__ __forceinline__ bool is_ghost(const Geom& g, int x, int y, int z) {
 }
 
 // state.f90:29-87, fixed gamma
-__global__ void k_phase_state(Geom g, PhaseArrays a, Ctrl* ctrl) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= g.ng) return;
+__device__ __forceinline__ void state_cell(const Geom& g, const PhaseArrays& a, Ctrl* ctrl,
+                                           long long i) {
   const long long n = g.ng;
   const double d = a.cons[i];
   const double u1 = a.u[i], u2 = a.u[n + i], u3 = a.u[2 * n + i];
@@ -1480,14 +1522,14 @@ __global__ void k_phase_state(Geom g, PhaseArrays a, Ctrl* ctrl) {
 }
 
 // velocity.f90:18-53
-__global__ void k_phase_velocity(Geom g, PhaseArrays a, Ctrl* ctrl) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= g.ng) return;
+__device__ __forceinline__ void velocity_cell(const Geom& g, const PhaseArrays& a, Ctrl* ctrl,
+                                              long long i) {
   const long long n = g.ng;
   double* c = a.cons;
   const double d = c[i];
+  const SharedDiv qd(d);
   double u[3];
-  for (int k = 0; k < 3; ++k) u[k] = c[(k + 1) * n + i] / d;
+  for (int k = 0; k < 3; ++k) u[k] = qd(c[(k + 1) * n + i]);
   int flag = 0;
   for (int k = 0; k < 3; ++k)
     if (fabs(u[k]) > g.vlimit) flag = 1;
@@ -1506,6 +1548,23 @@ __global__ void k_phase_velocity(Geom g, PhaseArrays a, Ctrl* ctrl) {
     atomicOr(&ctrl->flags, (unsigned)kFlagVlimit);
   }
   for (int k = 0; k < 3; ++k) a.u[k * n + i] = u[k];
+}
+
+__global__ void k_phase_state(Geom g, PhaseArrays a, Ctrl* ctrl) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i < g.ng) state_cell(g, a, ctrl, i);
+}
+__global__ void k_phase_velocity(Geom g, PhaseArrays a, Ctrl* ctrl) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i < g.ng) velocity_cell(g, a, ctrl, i);
+}
+// state() and velocity() in a row (four times a step): both look at their own cell
+// only, so the second finds the first's lines in L1
+__global__ void k_phase_state_velocity(Geom g, PhaseArrays a, Ctrl* ctrl) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= g.ng) return;
+  state_cell(g, a, ctrl, i);
+  velocity_cell(g, a, ctrl, i);
 }
 
 // courant.f90:19-23 (max over every cell, ghosts included)
@@ -1887,6 +1946,35 @@ __global__ void k_phase_faces(Geom g, PhaseArrays a, double* F) {
   }
 }
 
+// the end of flux(avg) after k_phase_tile: its results to the interior cells, and the
+// ghosts' (whose fluxes are zero) own update and floors (flux.f90:186-230).  save: the
+// cons before it to cons_old first (main.f90:327-333), which the flux left alone
+__global__ void k_phase_commit(Geom g, PhaseArrays a, Ctrl* ctrl, const double* out, int avg,
+                               int save) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= g.ng) return;
+  const long long n = g.ng;
+  const int x = (int)(i % g.nx), y = (int)((i / g.nx) % g.ny), z = (int)(i / g.sz);
+  if (save)
+    for (int k = 0; k < 5; ++k) a.cons_old[k * n + i] = a.cons[k * n + i];
+  if (!is_ghost(g, x, y, z)) {
+    for (int k = 0; k < 5; ++k) a.cons[k * n + i] = out[k * n + i];
+    return;
+  }
+  double v[5];
+  for (int k = 0; k < 5; ++k) {
+    const double c = a.cons[k * n + i];
+    v[k] = avg == 0 ? c : kHalf * (a.cons_old[k * n + i] + c);
+  }
+  floors(v[0], v[1], v[2], v[3], v[4], g.small_rho, g.small_eps);
+  bool bad = false;
+  for (int k = 0; k < 5; ++k) {
+    a.cons[k * n + i] = v[k];
+    if (!isfinite(v[k])) bad = true;
+  }
+  if (bad) atomicOr(&ctrl->flags, (unsigned)kFlagNonFinite);
+}
+
 __global__ void k_copy5(const double* src, double* dst, long long n) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= 5 * n) return;
@@ -2029,6 +2117,10 @@ cudaError_t phase_velocity(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream
   k_phase_velocity<<<nblk(g.ng), PB, 0, s>>>(g, a, ctrl);
   return cudaGetLastError();
 }
+cudaError_t phase_state_velocity(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream_t s) {
+  k_phase_state_velocity<<<nblk(g.ng), PB, 0, s>>>(g, a, ctrl);
+  return cudaGetLastError();
+}
 cudaError_t phase_courant(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream_t s) {
   k_phase_courant<<<nblk(g.ng), PB, 0, s>>>(g, a, ctrl);
   return cudaGetLastError();
@@ -2079,7 +2171,50 @@ cudaError_t phase_ghost(int nghost, const int32_t* dst, const int32_t* src, cons
   k_ghost_scatter<<<nblk(nghost), PB, 0, s>>>(nghost, dst, a.gtmp, a.cons, ng);
   return cudaGetLastError();
 }
-cudaError_t phase_flux(const Geom& g, PhaseArrays& a, Ctrl* ctrl, int avg, cudaStream_t s) {
+template <int AVG, int PM, bool THREED>
+static cudaError_t launch_phase_tile(const StageArgs& t, int ntiles, cudaStream_t s) {
+  const size_t smem = Shape0::SMEM_DOUBLES * sizeof(double);
+  const cudaError_t e = ensure_dyn_smem((const void*)k_phase_tile<AVG, PM, THREED>, smem);
+  if (e != cudaSuccess) return e;
+  k_phase_tile<AVG, PM, THREED><<<ntiles, Shape0::NT, smem, s>>>(t);
+  return cudaGetLastError();
+}
+template <int AVG>
+static cudaError_t launch_phase_tile(const Geom& g, const StageArgs& t, int ntiles,
+                                     cudaStream_t s) {
+  if (g.pow2) return g.threed ? launch_phase_tile<AVG, 1, true>(t, ntiles, s)
+                              : launch_phase_tile<AVG, 1, false>(t, ntiles, s);
+  return g.threed ? launch_phase_tile<AVG, 0, true>(t, ntiles, s)
+                  : launch_phase_tile<AVG, 0, false>(t, ntiles, s);
+}
+
+// With fixed gamma and no flux_ang the flux runs on the stage kernels' tiles (adindx
+// is gammafix in every cell then, as state() leaves it).  The kernels per cell and
+// face beside it pass 42 doubles of face states and 15 of fluxes per cell through
+// memory: 205 us per flux at 96^3 against 133 with the tiles and the commit.
+cudaError_t phase_flux(const Geom& g, PhaseArrays& a, Ctrl* ctrl, int avg, cudaStream_t s,
+                       bool save_old) {
+  if (!g.ang && !g.tab) {
+    StageArgs t{};
+    t.X = avg ? a.cons_old : a.cons;
+    t.Y = a.cons;
+    t.U = a.u;
+    t.P = a.p;
+    t.out = a.states;
+    t.ctrl = ctrl;
+    t.geom = a.geom;
+    t.tiles = a.tiles;
+    t.ncells_total = g.ng;
+    const cudaError_t e = avg ? launch_phase_tile<1>(g, t, a.ntiles, s)
+                              : launch_phase_tile<0>(g, t, a.ntiles, s);
+    if (e != cudaSuccess) return e;
+    k_phase_commit<<<nblk(g.ng), PB, 0, s>>>(g, a, ctrl, a.states, avg, save_old);
+    return cudaGetLastError();
+  }
+  if (save_old) {
+    const cudaError_t e = phase_copy_old(g, a, s);
+    if (e != cudaSuccess) return e;
+  }
   if (g.ang) {
     k_ang_to<<<nblk(g.ng), PB, 0, s>>>(g, a, avg);
     k_phase_states<true><<<nblk(g.ng), PB, 0, s>>>(g, a, ctrl);

@@ -1,4 +1,5 @@
-"""The tiled stage kernels at the edges of their tiles, against the oracle.
+"""The tiled stage kernels (and the per-phase flux on them) at the edges of their
+tiles, against the oracle.
 
 Interior sizes of one cell, one short of, at and one beyond a tile's columns (32 x 8;
 32 x 6 with flux_ang) and of a z chunk, with and without walls and with a cell
@@ -49,5 +50,18 @@ def test_tile_edges_with_flux_ang(n):
     o, g = make_pair(st)
     step_both(o, g, 4)
     assert g.status()[1] == 1 and np.isfinite(g.download()[0]).all()
+    o.close()
+    g.close()
+
+
+@pytest.mark.parametrize("n", [(1, 1, 2), (33, 9, 3), (32, 8, 2), (65, 7, 9), (33, 9, 2), (5, 17, 1)])
+@pytest.mark.parametrize("walls,dx", [((1,) * 6, 1.0 / 16), ((0, 1, 1, 0, 0, 1), 0.07)])
+def test_tile_edges_per_phase(n, walls, dx):
+    """The per-phase path's flux on the same tiles, on the reference's arrays."""
+    nz = n[2] + 4 if n[2] > 1 else 1
+    st = small_random_box(nx=n[0] + 4, ny=n[1] + 4, nz=nz, walls=walls, dx=dx, seed=2 + sum(n))
+    o, g = make_pair(st, phase_only=True)
+    step_both(o, g, 3)
+    assert g.status()[1] == 0
     o.close()
     g.close()
