@@ -1152,6 +1152,8 @@ static int fwd_step(bx_adj* A, const double* X, int nsrc, double dt, double* Y,
   StageArgs a{};
   a.ctrl = h->d_ctrl;
   a.geom = h->d_geom;
+  a.single = 1;
+  a.g0 = h->g;
   a.tiles = h->d_tiles;
   a.ncells_total = h->g.ng;
   a.nsrc = nsrc;
@@ -1160,11 +1162,11 @@ static int fwd_step(bx_adj* A, const double* X, int nsrc, double dt, double* Y,
   a.X = X;
   a.Y = nullptr;
   a.out = c1out ? c1out : A->W1;
-  ACK(launch_stage(0, h->g.pow2 ? 1 : 0, h->g.threed != 0, a, h->ntiles, h->stream));
+  ACK(launch_stage(0, h->g.pow2 ? 1 : 0, h->g.threed != 0, a, h->ntiles, h->stream, h->launch_shape()));
   if (stage0_only) return BX_OK;
   a.Y = a.out;
   a.out = Y;
-  ACK(launch_stage(1, h->g.pow2 ? 1 : 0, h->g.threed != 0, a, h->ntiles, h->stream));
+  ACK(launch_stage(1, h->g.pow2 ? 1 : 0, h->g.threed != 0, a, h->ntiles, h->stream, h->launch_shape()));
   return BX_OK;
 }
 
@@ -1735,6 +1737,8 @@ int bx_adj_forward(bx_adj* A, const double* cons0, double* consT, int32_t frozen
     StageArgs a{};
     a.ctrl = h->d_ctrl;
     a.geom = h->d_geom;
+  a.single = 1;
+  a.g0 = h->g;
     a.tiles = h->d_tiles;
     a.ncells_total = g.ng;
     a.nsrc = nsrc;
@@ -1746,10 +1750,10 @@ int bx_adj_forward(bx_adj* A, const double* cons0, double* consT, int32_t frozen
     }
     a.X = cur;
     a.out = (!frozen && A->c1pool) ? A->c1pool + k * n5 : A->W1;
-    ACK(launch_stage(0, g.pow2 ? 1 : 0, g.threed != 0, a, h->ntiles, s));
+    ACK(launch_stage(0, g.pow2 ? 1 : 0, g.threed != 0, a, h->ntiles, s, h->launch_shape()));
     a.Y = a.out;
     a.out = out;
-    ACK(launch_stage(1, g.pow2 ? 1 : 0, g.threed != 0, a, h->ntiles, s));
+    ACK(launch_stage(1, g.pow2 ? 1 : 0, g.threed != 0, a, h->ntiles, s, h->launch_shape()));
     if (!given_dt)
       ACK(launch_next_run(h->d_ctrl, k + 1 < A->nsteps ? A->d_dts + k + 1 : nullptr, s));
     if (hb >= 0) {

@@ -191,6 +191,8 @@ static int create_handle(const bx_params* params, bx_handle** out, bool lean) {
   const int per_sm = std::max(1, stage_blocks_per_sm(1, h->g.pow2, h->g.threed, h->shape));
   std::vector<Tile> tiles = make_tiles(h->g, 0, sms * per_sm, 0, h->shape);
   h->ntiles = (int)tiles.size();
+  // one tile per SM at most: kWideShape
+  h->wide = h->shape == 0 && h->ntiles <= sms;
   CKC(dalloc((void**)&h->d_tiles, tiles.size() * sizeof(Tile)));
   CKC(cudaMemcpy(h->d_tiles, tiles.data(), tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice));
   h->pa.geom = h->d_geom;
@@ -709,6 +711,8 @@ static int fused_launch(bx_handle* h) {
   StageArgs a{};
   a.ctrl = h->d_ctrl;
   a.geom = h->d_geom;
+  a.single = 1;
+  a.g0 = h->g;
   a.tiles = h->d_tiles;
   a.ncells_total = h->g.ng;
   a.eos = h->pa.eos;
@@ -725,11 +729,11 @@ static int fused_launch(bx_handle* h) {
   a.Y = nullptr;
   a.out = h->buf[Y];
   if (h->prof) CK(cudaEventRecord(h->ev[0], h->stream));
-  CK(launch_stage(0, p2, t3, a, h->ntiles, h->stream, h->shape));
+  CK(launch_stage(0, p2, t3, a, h->ntiles, h->stream, h->launch_shape()));
   if (h->prof) CK(cudaEventRecord(h->ev[1], h->stream));
   a.Y = h->buf[Y];
   a.out = h->buf[Z];
-  CK(launch_stage(1, p2, t3, a, h->ntiles, h->stream, h->shape));
+  CK(launch_stage(1, p2, t3, a, h->ntiles, h->stream, h->launch_shape()));
   if (h->prof) CK(cudaEventRecord(h->ev[2], h->stream));
   CK(launch_end(h->d_ctrl, 1, h->stream));
   h->launches += 4;
@@ -947,6 +951,8 @@ static int host_io_enqueue(bx_handle* h, const double* cons_in, double* cons_out
   StageArgs a{};
   a.ctrl = h->d_ctrl;
   a.geom = h->d_geom;
+  a.single = 1;
+  a.g0 = h->g;
   a.ncells_total = n;
   a.nsrc = h->nsrc;
   a.U = h->pa.u;
@@ -1259,6 +1265,8 @@ static int fused_run(bx_handle* h, double endtime, int64_t nsteps, int64_t* take
   StageArgs a{};
   a.ctrl = h->d_ctrl;
   a.geom = h->d_geom;
+  a.single = 1;
+  a.g0 = h->g;
   a.tiles = h->d_tiles;
   a.ncells_total = g.ng;
   a.eos = h->pa.eos;
@@ -1274,10 +1282,10 @@ static int fused_run(bx_handle* h, double endtime, int64_t nsteps, int64_t* take
       a.X = h->buf[cur];
       a.Y = nullptr;
       a.out = h->buf[(cur + 1) % 3];
-      if (e == cudaSuccess) e = launch_stage(0, p2, t3, a, h->ntiles, s, h->shape);
+      if (e == cudaSuccess) e = launch_stage(0, p2, t3, a, h->ntiles, s, h->launch_shape());
       a.Y = h->buf[(cur + 1) % 3];
       a.out = h->buf[(cur + 2) % 3];
-      if (e == cudaSuccess) e = launch_stage(1, p2, t3, a, h->ntiles, s, h->shape);
+      if (e == cudaSuccess) e = launch_stage(1, p2, t3, a, h->ntiles, s, h->launch_shape());
       if (e == cudaSuccess)
         e = k + 1 < K ? launch_next_batch(h->d_ctrl, 1, s) : launch_end_batch(h->d_ctrl, 1, s);
       if (e != cudaSuccess) return e;

@@ -45,6 +45,8 @@ struct bx_handle {
   // set (update_eligible)
   bool fusable = false;
   int shape = 0;  // stage-kernel tile shape of the single-grid launches
+  bool wide = false;  // shape 0 on a grid of at most one tile per SM: kWideShape
+  int launch_shape() const { return wide && !gforce_set ? bx::kWideShape : shape; }
   bool gforce_set = false;
   uint32_t status = 0;
   int last_path = 0;

@@ -117,6 +117,14 @@ using Shape1 = TileShape<16, 16>;
 // per 96^3 step; 224 threads get the same 128 registers)
 using Shape2 = TileShape<32, 6, 1, 192>;
 using Shape3 = TileShape<32, 6, 2, 192>;
+// grids of at most one tile per SM, where a second block per SM has nothing to do:
+// twice the threads on a tile, so those without a column take the halo's primitives
+// and the rim's states and faces beside the columns' own (two rounds instead of
+// three; 32^3 28.4 against 26.6 us per step, 512-cell tube 15.6 against 14.3; beyond
+// one tile per SM two 256-thread blocks hide each other's barriers);
+// kWideShape's extents are shape 0's
+using Shape4 = TileShape<32, 8, 0, 512>;
+constexpr int kWideShape = 4;
 constexpr int kNumShapes = 2;  // the shapes the batched autotuner chooses among
 // the x and y extents of tile shape `shape`
 inline int shape_tx(int shape) {
@@ -127,7 +135,11 @@ inline int shape_ty(int shape) {
 }
 
 inline int shape_threads(int shape) {
-  return shape == 3 ? Shape3::NT : shape == 2 ? Shape2::NT : shape == 1 ? Shape1::NT : Shape0::NT;
+  return shape == 4   ? Shape4::NT
+         : shape == 3 ? Shape3::NT
+         : shape == 2 ? Shape2::NT
+         : shape == 1 ? Shape1::NT
+                      : Shape0::NT;
 }
 
 // ghost-fill tables: per ghost (index order), destination cell, source cell and
@@ -174,6 +186,8 @@ struct StageArgs {
                      // own cells (the velocity state() reads at the step's end)
   Ctrl* ctrl;        // per box control blocks
   const Geom* geom;  // per box geometry (device)
+  int single;        // one grid: its geometry is g0
+  Geom g0;
   const Tile* tiles;
   long long ncells_total;  // plane stride of the pooled buffers
   int nsrc;                // > 0: sources the input is short of; 0: per box (Ctrl::nsrc)

@@ -16,7 +16,7 @@ from tests.helpers import make_pair, small_random_box, step_both
 pytestmark = pytest.mark.gpu
 
 SIZES = [(1, 1, 2), (2, 8, 3), (31, 9, 2), (33, 7, 5), (32, 8, 2), (65, 17, 3), (64, 1, 2),
-         (3, 41, 9)]
+         (3, 41, 9), (75, 61, 47)]
 
 
 @pytest.mark.parametrize("n", SIZES)
