@@ -192,6 +192,7 @@ static int create_handle(const bx_params* params, bx_handle** out, bool lean) {
   std::vector<Tile> tiles = make_tiles(h->g, 0, sms * per_sm, 0, h->shape);
   h->ntiles = (int)tiles.size();
   // one tile per SM at most: kWideShape
+  h->sms = sms;
   h->wide = h->shape == 0 && h->ntiles <= sms;
   CKC(dalloc((void**)&h->d_tiles, tiles.size() * sizeof(Tile)));
   CKC(cudaMemcpy(h->d_tiles, tiles.data(), tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice));
@@ -852,12 +853,16 @@ static int host_io_setup(bx_handle* h) {
   if (!h->slabs.empty()) return BX_OK;
   const Geom& g = h->g;
   const long long n = g.ng;
-  // thin chunks (about 64 slabs, at least 2 planes each): a slab's copy back
-  // can start once the planes up to four beyond it are in (256^3 measured
-  // 15.8 ms per step with 64 slabs, 17.0 with 32, 21.1 with the 8 chunks of
-  // the stage launches)
+  // thin chunks, so that a slab's copy back can start once the planes up to four
+  // beyond it are in: about 64 slabs (256^3 measured 15.8 ms per step with 64, 17.0
+  // with 32, 21.1 with the 8 chunks of the stage launches), but no thinner than 2^17
+  // cells (5 MB, 0.1 ms of copying) up to 8 planes, below which a slab's ten launches
+  // and events cost more than its copies: per step with 2, 4, 8 and 16 planes 3.23,
+  // 2.83, 2.76 and 2.95 ms at 128^3, 1.26, 1.00, 0.88 and 0.92 at 64^3
   const int naz = g.az1 - g.az0;
-  const std::vector<Tile> tiles = make_tiles(g, 0, 1, std::max(2, (naz + 63) / 64));
+  const int thin = (int)std::min<long long>(8, ((1ll << 17) + g.sz - 1) / g.sz);
+  const int zc = std::max({2, thin, (naz + 63) / 64});
+  const std::vector<Tile> tiles = make_tiles(g, 0, 1, zc);
   CK(cudaMalloc((void**)&h->d_io_tiles, tiles.size() * sizeof(Tile)));
   CK(cudaMemcpy(h->d_io_tiles, tiles.data(), tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice));
   struct Chunk {
@@ -985,7 +990,7 @@ static int host_io_enqueue(bx_handle* h, const double* cons_in, double* cons_out
       StageArgs aj = a;
       aj.tiles = h->d_io_tiles + sl.t0;
       aj.out = h->buf[Yi];
-      CK(launch_stage(0, p2, t3, aj, sl.nt, s));
+      CK(launch_stage(0, p2, t3, aj, sl.nt, s, h->io_shape(sl.nt)));
       h->launches += 1;
     }
     CK(cudaEventRecord(ev_s0[k], s));
@@ -999,7 +1004,7 @@ static int host_io_enqueue(bx_handle* h, const double* cons_in, double* cons_out
       aj.tiles = h->d_io_tiles + sl.t0;
       aj.Y = h->buf[Yi];
       aj.out = h->buf[Zi];
-      CK(launch_stage(1, p2, t3, aj, sl.nt, sj));
+      CK(launch_stage(1, p2, t3, aj, sl.nt, sj, h->io_shape(sl.nt)));
       CK(cudaEventRecord(ev_st1[j], sj));
       if (tp) CK(cudaEventRecord(tev(j, 3), sj));
       CK(cudaStreamWaitEvent(cs, ev_st1[j], 0));
