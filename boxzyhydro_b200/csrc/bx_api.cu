@@ -199,6 +199,8 @@ static int create_handle(const bx_params* params, bx_handle** out, bool lean) {
   h->pa.geom = h->d_geom;
   h->pa.tiles = h->d_tiles;
   h->pa.ntiles = h->ntiles;
+  h->pa.nghost = h->nghost;
+  h->pa.gdst = h->d_dst;
   CKC(dalloc((void**)&h->d_ctrl, sizeof(Ctrl)));
   CKC(cudaMallocHost((void**)&h->h_ctrl, sizeof(Ctrl)));
   std::memset(&h->clock, 0, sizeof(Ctrl));
@@ -350,15 +352,15 @@ int bx_upload(bx_handle* h, const double* cons, const double* u, const double* p
   // a state the fused stages reproduce exactly (as left by a previous step)
   // continues on them; anything else starts on the per-phase kernels
   if (h->eligible) {
-    if (int r = pull_clock(h)) return r;
-    h->clock.flags = 0;
-    if (int r = push_clock(h)) return r;
+    CK(cudaMemsetAsync(&h->d_ctrl->flags, 0, sizeof(h->d_ctrl->flags), s));
     CK(check_clean(h->g, h->pa, h->nghost, h->d_dst, h->d_src2, h->d_sgn2, h->d_ctrl, s));
     h->launches += 2;
     if (int r = pull_clock(h)) return r;
     const bool clean = !(h->clock.flags & kFlagNotClean);
-    h->clock.flags = 0;
-    if (int r = push_clock(h)) return r;
+    if (h->clock.flags) {
+      h->clock.flags = 0;
+      if (int r = push_clock(h)) return r;
+    }
     if (clean) {
       // adindx = gammafix is what state() leaves; set it like the other path does
       return enter_fused(h);
@@ -381,15 +383,15 @@ int bx_upload_conserved(bx_handle* h, const double* cons) {
   h->launches += 2;
   h->mode = 0;
   if (h->eligible) {
-    if (int r = pull_clock(h)) return r;
-    h->clock.flags = 0;
-    if (int r = push_clock(h)) return r;
+    CK(cudaMemsetAsync(&h->d_ctrl->flags, 0, sizeof(h->d_ctrl->flags), s));
     CK(check_clean(h->g, h->pa, h->nghost, h->d_dst, h->d_src2, h->d_sgn2, h->d_ctrl, s));
     h->launches += 2;
     if (int r = pull_clock(h)) return r;
     const bool clean = !(h->clock.flags & kFlagNotClean);
-    h->clock.flags = 0;
-    if (int r = push_clock(h)) return r;
+    if (h->clock.flags) {
+      h->clock.flags = 0;
+      if (int r = push_clock(h)) return r;
+    }
     if (clean) return enter_fused(h);
   }
   return bx_adindx_fill(h);
@@ -422,7 +424,6 @@ int bx_download(bx_handle* h, double* cons, double* u, double* p) {
 
 int bx_set_clock(bx_handle* h, double time, double dtold, int64_t step) {
   CHECK_H();
-  if (int r = pull_clock(h)) return r;
   h->clock.time = time;
   h->clock.dtold = dtold;
   h->clock.step = step;

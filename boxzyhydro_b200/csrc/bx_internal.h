@@ -234,6 +234,8 @@ struct PhaseArrays {
   const Geom* geom; // the grid on the device, and its stage-kernel tiles (the flux
   const Tile* tiles;// with fixed gamma)
   int ntiles;
+  int nghost;       // the ghost cells, in index order
+  const int32_t* gdst;
 };
 
 cudaError_t phase_state(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream_t s);
@@ -244,7 +246,8 @@ cudaError_t phase_source(const Geom& g, PhaseArrays& a, Ctrl* ctrl, double mult,
 cudaError_t phase_calc_gforce(const Geom& g, const double* phi, double* gforce, cudaStream_t s);
 cudaError_t phase_ghost(int nghost, const int32_t* dst, const int32_t* src, const uint8_t* sgn,
                         PhaseArrays& a, long long ng, cudaStream_t s);
-// save_old: phase_copy_old first
+// save_old: phase_copy_old first.  With fixed gamma a's cons, states and (save_old)
+// cons_old change places
 cudaError_t phase_flux(const Geom& g, PhaseArrays& a, Ctrl* ctrl, int avg, cudaStream_t s,
                        bool save_old = false);
 cudaError_t phase_courant_finish(Ctrl* ctrl, cudaStream_t s);

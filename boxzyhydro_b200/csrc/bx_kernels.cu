@@ -1961,30 +1961,22 @@ __global__ void k_phase_faces(Geom g, PhaseArrays a, double* F) {
   }
 }
 
-// the end of flux(avg) after k_phase_tile: its results to the interior cells, and the
-// ghosts' (whose fluxes are zero) own update and floors (flux.f90:186-230).  save: the
-// cons before it to cons_old first (main.f90:327-333), which the flux left alone
-__global__ void k_phase_commit(Geom g, PhaseArrays a, Ctrl* ctrl, const double* out, int avg,
-                               int save) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= g.ng) return;
-  const long long n = g.ng;
-  const int x = (int)(i % g.nx), y = (int)((i / g.nx) % g.ny), z = (int)(i / g.sz);
-  if (save)
-    for (int k = 0; k < 5; ++k) a.cons_old[k * n + i] = a.cons[k * n + i];
-  if (!is_ghost(g, x, y, z)) {
-    for (int k = 0; k < 5; ++k) a.cons[k * n + i] = out[k * n + i];
-    return;
-  }
+// the ghosts' part of flux(avg) beside k_phase_tile (their fluxes are zero): the update
+// and floors (flux.f90:186-230), from cons to out
+__global__ void k_phase_ghost_update(int nghost, const int32_t* dst, Geom g, const double* cons,
+                                     const double* cons_old, double* out, Ctrl* ctrl, int avg) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= nghost) return;
+  const long long i = dst[j], n = g.ng;
   double v[5];
   for (int k = 0; k < 5; ++k) {
-    const double c = a.cons[k * n + i];
-    v[k] = avg == 0 ? c : kHalf * (a.cons_old[k * n + i] + c);
+    const double c = cons[k * n + i];
+    v[k] = avg == 0 ? c : kHalf * (cons_old[k * n + i] + c);
   }
   floors(v[0], v[1], v[2], v[3], v[4], g.small_rho, g.small_eps);
   bool bad = false;
   for (int k = 0; k < 5; ++k) {
-    a.cons[k * n + i] = v[k];
+    out[k * n + i] = v[k];
     if (!isfinite(v[k])) bad = true;
   }
   if (bad) atomicOr(&ctrl->flags, (unsigned)kFlagNonFinite);
@@ -2206,7 +2198,9 @@ static cudaError_t launch_phase_tile(const Geom& g, const StageArgs& t, int ntil
 // With fixed gamma and no flux_ang the flux runs on the stage kernels' tiles (adindx
 // is gammafix in every cell then, as state() leaves it).  The kernels per cell and
 // face beside it pass 42 doubles of face states and 15 of fluxes per cell through
-// memory: 205 us per flux at 96^3 against 133 with the tiles and the commit.
+// memory: 205 us per flux at 96^3 against 121 with the tiles.  The tiles cannot write
+// in place (their halos read their neighbours' cells), so the result's planes become
+// cons, and with save_old the planes it came from cons_old: no copies.
 cudaError_t phase_flux(const Geom& g, PhaseArrays& a, Ctrl* ctrl, int avg, cudaStream_t s,
                        bool save_old) {
   if (!g.ang && !g.tab) {
@@ -2223,7 +2217,11 @@ cudaError_t phase_flux(const Geom& g, PhaseArrays& a, Ctrl* ctrl, int avg, cudaS
     const cudaError_t e = avg ? launch_phase_tile<1>(g, t, a.ntiles, s)
                               : launch_phase_tile<0>(g, t, a.ntiles, s);
     if (e != cudaSuccess) return e;
-    k_phase_commit<<<nblk(g.ng), PB, 0, s>>>(g, a, ctrl, a.states, avg, save_old);
+    if (a.nghost > 0)
+      k_phase_ghost_update<<<nblk(a.nghost), PB, 0, s>>>(a.nghost, a.gdst, g, a.cons, a.cons_old,
+                                                         a.states, ctrl, avg);
+    std::swap(a.cons, a.states);                    // states: the cons before the flux
+    if (save_old) std::swap(a.cons_old, a.states);
     return cudaGetLastError();
   }
   if (save_old) {
