@@ -1157,6 +1157,7 @@ static int fwd_step(bx_adj* A, const double* X, int nsrc, double dt, double* Y,
   a.tiles = h->d_tiles;
   a.ncells_total = h->g.ng;
   a.nsrc = nsrc;
+  a.after = 1;
   a.U = A->P;  // the primitives are rebuilt by every reverse stage
   k_set_clock<<<1, 1, 0, h->stream>>>(h->d_ctrl, dt, 1);
   a.X = X;
@@ -1742,6 +1743,7 @@ int bx_adj_forward(bx_adj* A, const double* cons0, double* consT, int32_t frozen
     a.tiles = h->d_tiles;
     a.ncells_total = g.ng;
     a.nsrc = nsrc;
+    a.after = hb < 0;  // else the input of a copy on another stream
     a.U = A->P;
     if (given_dt) {
       k_set_clock<<<1, 1, 0, s>>>(h->d_ctrl, A->dts[k], 1);

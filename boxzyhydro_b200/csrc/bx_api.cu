@@ -690,7 +690,7 @@ static int phase_step(bx_handle* h) {
   CK(phase_state(g, a, c, s));
   CK(cudaMemsetAsync(&c->rate_bits, 0, sizeof(unsigned long long), s));
   CK(phase_courant(g, a, c, s));
-  CK(launch_dt(c, 1, s));
+  CK(launch_dt(c, 1, s, true));
   CK(phase_source(g, a, c, 0.5, s));   // source(time,0) with dt/2
   if (int r = ghost2(h)) return r;
   CK(phase_state_velocity(g, a, c, s));
@@ -703,7 +703,7 @@ static int phase_step(bx_handle* h) {
   CK(phase_source(g, a, c, 0.5, s));   // source(time+dt,1) with dt/2
   if (int r = ghost2(h)) return r;
   CK(phase_state_velocity(g, a, c, s));
-  CK(launch_end(c, 1, s));
+  CK(launch_end(c, 1, s, true));
   h->launches += 22 + (g.ang || g.tab ? 3 : 0);
   return BX_OK;
 }
@@ -726,7 +726,8 @@ static int fused_launch(bx_handle* h) {
   a.G = h->gforce_set ? h->pa.gforce : nullptr;
   a.UC = h->pa.cons_old;
   const bool p2 = h->g.pow2 != 0, t3 = h->g.threed != 0;
-  CK(launch_dt(h->d_ctrl, 1, h->stream));
+  a.after = !h->prof;  // with events between the launches each is timed by itself
+  CK(launch_dt(h->d_ctrl, 1, h->stream, a.after));
   a.X = h->buf[X];
   a.Y = nullptr;
   a.out = h->buf[Y];
@@ -737,7 +738,7 @@ static int fused_launch(bx_handle* h) {
   a.out = h->buf[Z];
   CK(launch_stage(1, p2, t3, a, h->ntiles, h->stream, h->launch_shape()));
   if (h->prof) CK(cudaEventRecord(h->ev[2], h->stream));
-  CK(launch_end(h->d_ctrl, 1, h->stream));
+  CK(launch_end(h->d_ctrl, 1, h->stream, a.after));
   h->launches += 4;
   return BX_OK;
 }
@@ -1279,6 +1280,7 @@ static int fused_run(bx_handle* h, double endtime, int64_t nsteps, int64_t* take
   a.U = h->pa.u;
   a.G = h->gforce_set ? h->pa.gforce : nullptr;
   a.UC = h->pa.cons_old;
+  a.after = 1;
   const bool p2 = g.pow2 != 0, t3 = g.threed != 0;
   auto enqueue = [&]() -> cudaError_t {
     int cur = cur0;

@@ -491,6 +491,7 @@ static int enqueue_steps(bx_batch* b, int nsteps) {
   for (int k = 0; k < nsteps; ++k) {
     const int X = c, Y = (c + 1) % 3, Z = (c + 2) % 3;
     b->step_x[k] = X;
+    a.after = 1;
     if (k == 0) BCK(launch_dt_batch(b->d_ctrl, b->nbox, b->stream));
     a.X = b->buf[X];
     a.Y = nullptr;

@@ -190,6 +190,7 @@ struct StageArgs {
   Geom g0;
   const Tile* tiles;
   long long ncells_total;  // plane stride of the pooled buffers
+  int after;               // the launch may start before the stream's last kernel is through
   int nsrc;                // > 0: sources the input is short of; 0: per box (Ctrl::nsrc)
   EosDev eos;              // the tables of the tabulated EOS (tile shape 2 only)
 };
@@ -208,14 +209,14 @@ int stage_blocks_per_sm(int stage, int pm, bool threed, int shape = 0);
 // pm: 1 = every box has power-of-two spacings, 0 = otherwise
 cudaError_t launch_stage(int stage, int pm, bool threed, const StageArgs& a, int ntiles,
                          cudaStream_t s, int shape = 0);
-cudaError_t launch_dt(Ctrl* ctrl, int nbox, cudaStream_t s);
+cudaError_t launch_dt(Ctrl* ctrl, int nbox, cudaStream_t s, bool after = false);
 // one box: launch_dt with the step's dt into *record; launch_end and, if record is not
 // null, the next step's launch_begin_run
 cudaError_t launch_begin_run(Ctrl* ctrl, double* record, cudaStream_t s);
 cudaError_t launch_next_run(Ctrl* ctrl, double* record, cudaStream_t s);
 // launch_end_batch, then the next step's launch_dt_batch
 cudaError_t launch_next_batch(Ctrl* ctrl, int nbox, cudaStream_t s);
-cudaError_t launch_end(Ctrl* ctrl, int nbox, cudaStream_t s);
+cudaError_t launch_end(Ctrl* ctrl, int nbox, cudaStream_t s, bool after = false);
 
 // phase kernels (one reference subroutine each, full arrays)
 struct PhaseArrays {

@@ -27,6 +27,7 @@
 #include <utility>
 
 #include "bx_internal.h"
+#include "bx_launch.cuh"
 #include "bx_math.cuh"
 
 namespace bx {
@@ -97,13 +98,13 @@ __device__ __forceinline__ void get_gamma2(const EosDev& e, double& eps, double 
   }
 }
 
-// Loads of the stage inputs: through the read-only path when the planes stay
-// unchanged for the whole launch (one launch per stage), from L2 (cg) in the
-// persistent batched kernel, whose other blocks write planes that this block
-// reads later in the same launch.
+// Loads of the stage inputs: plain ones where the launch waits for the one before it
+// (grid_wait; not the read-only path, whose data may not change once a kernel has
+// started), from L2 (cg) in the persistent batched kernel, whose other blocks write
+// planes that this block reads later in the same launch.
 template <bool CG = false>
 __device__ __forceinline__ double ldg(const double* p) {
-  return CG ? __ldcg(p) : __ldg(p);
+  return CG ? __ldcg(p) : __ldca(p);
 }
 
 // donor of a coordinate along one axis for a face ghost (fused path)
@@ -1119,8 +1120,6 @@ __global__ void __launch_bounds__(ShapeSel<SH>::type::NT, ShapeSel<SH>::type::NT
   // so their loads do not wait for the tile's (0.6 us a step on small grids)
   const Tile t = a.tiles[blockIdx.x];
   Ctrl* C = a.ctrl + (a.single ? 0 : t.box);
-  const int active = C->active, cn = C->nsrc;
-  const double dt = C->dt;
   if (a.single) {
     const int* src = reinterpret_cast<const int*>(&a.g0);
     if (threadIdx.x < sizeof(Geom) / sizeof(int))
@@ -1128,6 +1127,10 @@ __global__ void __launch_bounds__(ShapeSel<SH>::type::NT, ShapeSel<SH>::type::NT
   } else if (threadIdx.x == 0) {
     sg = a.geom[t.box];
   }
+  grid_wait();
+  grid_release();
+  const int active = C->active, cn = C->nsrc;
+  const double dt = C->dt;
   __syncthreads();
   if (!active) return;
   const int nsrc = a.nsrc > 0 ? a.nsrc : cn;
@@ -1144,6 +1147,8 @@ __global__ void __launch_bounds__(Shape0::NT, 2) k_phase_tile(StageArgs a) {
   __shared__ unsigned red_flags[Shape0::NT / 32];
   const Tile t = a.tiles[blockIdx.x];
   if (threadIdx.x == 0) sg = *a.geom;
+  grid_wait();
+  grid_release();
   __syncthreads();
   stage_tile<Shape0, AVG, PM == 1, THREED, false, false, true>(a, t, sg, a.ctrl, a.ctrl->dt, 0, sm,
                                                                red_rate, red_flags);
@@ -1331,8 +1336,8 @@ static cudaError_t launch_stage_t(const StageArgs& a, int ntiles, cudaStream_t s
   cudaError_t e = ensure_dyn_smem((const void*)k_stage<STAGE, PM, THREED, GRAV, SH>, smem);
   if (e != cudaSuccess) return e;
   if (ntiles <= 0) return cudaSuccess;
-  k_stage<STAGE, PM, THREED, GRAV, SH><<<ntiles, ShapeSel<SH>::type::NT, smem, s>>>(a);
-  return cudaGetLastError();
+  return launch_after(a.after, k_stage<STAGE, PM, THREED, GRAV, SH>, ntiles,
+                      ShapeSel<SH>::type::NT, smem, s, a);
 }
 
 template <int STAGE, bool GRAV, int SH>
@@ -1406,10 +1411,14 @@ __device__ __forceinline__ void clock_end(Ctrl& c) {
   c.time = c.time + dt;
 }
 __global__ void k_dt(Ctrl* ctrl, int n) {
+  grid_wait();
+  grid_release();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b < n) clock_begin(ctrl[b]);
 }
 __global__ void k_end(Ctrl* ctrl, int n) {
+  grid_wait();
+  grid_release();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b < n) clock_end(ctrl[b]);
 }
@@ -1423,12 +1432,16 @@ __global__ void k_begin_run(Ctrl* c, double* record) {
   *record = c->dt;
 }
 __global__ void k_next_run(Ctrl* c, double* record) {
+  grid_wait();
+  grid_release();
   clock_end(*c);
   if (!record) return;
   clock_begin(*c);
   *record = c->dt;
 }
 __global__ void k_next_batch(Ctrl* ctrl, int n) {
+  grid_wait();
+  grid_release();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n) return;
   box_end_step(ctrl[b]);
@@ -1438,43 +1451,41 @@ __global__ void k_next_batch(Ctrl* ctrl, int n) {
 // batched boxes: as k_dt/k_end, plus the saved clock and the trip of a box
 // whose step raised a guard (its planes then keep the step's input)
 __global__ void k_dt_batch(Ctrl* ctrl, int n) {
+  grid_wait();
+  grid_release();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n) return;
   box_begin_step(ctrl[b]);
 }
 __global__ void k_end_batch(Ctrl* ctrl, int n) {
+  grid_wait();
+  grid_release();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n) return;
   box_end_step(ctrl[b]);
 }
 cudaError_t launch_dt_batch(Ctrl* ctrl, int nbox, cudaStream_t s) {
-  k_dt_batch<<<(nbox + 127) / 128, 128, 0, s>>>(ctrl, nbox);
-  return cudaGetLastError();
+  return launch_after(true, k_dt_batch, (nbox + 127) / 128, 128, 0, s, ctrl, nbox);
 }
 cudaError_t launch_end_batch(Ctrl* ctrl, int nbox, cudaStream_t s) {
-  k_end_batch<<<(nbox + 127) / 128, 128, 0, s>>>(ctrl, nbox);
-  return cudaGetLastError();
+  return launch_after(true, k_end_batch, (nbox + 127) / 128, 128, 0, s, ctrl, nbox);
 }
 
-cudaError_t launch_dt(Ctrl* ctrl, int nbox, cudaStream_t s) {
-  k_dt<<<(nbox + 127) / 128, 128, 0, s>>>(ctrl, nbox);
-  return cudaGetLastError();
+cudaError_t launch_dt(Ctrl* ctrl, int nbox, cudaStream_t s, bool after) {
+  return launch_after(after, k_dt, (nbox + 127) / 128, 128, 0, s, ctrl, nbox);
 }
 cudaError_t launch_begin_run(Ctrl* ctrl, double* record, cudaStream_t s) {
   k_begin_run<<<1, 1, 0, s>>>(ctrl, record);
   return cudaGetLastError();
 }
 cudaError_t launch_next_run(Ctrl* ctrl, double* record, cudaStream_t s) {
-  k_next_run<<<1, 1, 0, s>>>(ctrl, record);
-  return cudaGetLastError();
+  return launch_after(true, k_next_run, 1, 1, 0, s, ctrl, record);
 }
 cudaError_t launch_next_batch(Ctrl* ctrl, int nbox, cudaStream_t s) {
-  k_next_batch<<<(nbox + 127) / 128, 128, 0, s>>>(ctrl, nbox);
-  return cudaGetLastError();
+  return launch_after(true, k_next_batch, (nbox + 127) / 128, 128, 0, s, ctrl, nbox);
 }
-cudaError_t launch_end(Ctrl* ctrl, int nbox, cudaStream_t s) {
-  k_end<<<(nbox + 127) / 128, 128, 0, s>>>(ctrl, nbox);
-  return cudaGetLastError();
+cudaError_t launch_end(Ctrl* ctrl, int nbox, cudaStream_t s, bool after) {
+  return launch_after(after, k_end, (nbox + 127) / 128, 128, 0, s, ctrl, nbox);
 }
 
 // ------------------------------------------------------------------ phase kernels
@@ -1566,16 +1577,22 @@ __device__ __forceinline__ void velocity_cell(const Geom& g, const PhaseArrays& 
 }
 
 __global__ void k_phase_state(Geom g, PhaseArrays a, Ctrl* ctrl) {
+  grid_wait();
+  grid_release();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i < g.ng) state_cell(g, a, ctrl, i);
 }
 __global__ void k_phase_velocity(Geom g, PhaseArrays a, Ctrl* ctrl) {
+  grid_wait();
+  grid_release();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i < g.ng) velocity_cell(g, a, ctrl, i);
 }
 // state() and velocity() in a row (four times a step): both look at their own cell
 // only, so the second finds the first's lines in L1
 __global__ void k_phase_state_velocity(Geom g, PhaseArrays a, Ctrl* ctrl) {
+  grid_wait();
+  grid_release();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= g.ng) return;
   state_cell(g, a, ctrl, i);
@@ -1584,6 +1601,8 @@ __global__ void k_phase_state_velocity(Geom g, PhaseArrays a, Ctrl* ctrl) {
 
 // courant.f90:19-23 (max over every cell, ghosts included)
 __global__ void k_phase_courant(Geom g, PhaseArrays a, Ctrl* ctrl) {
+  grid_wait();
+  grid_release();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long n = g.ng;
   double r = 0.0;
@@ -1680,6 +1699,8 @@ __global__ void k_phase_courant_finish(Ctrl* ctrl) {
 
 // source.f90:148-191 (interior cells)
 __global__ void k_phase_source(Geom g, PhaseArrays a, Ctrl* ctrl, double mult) {
+  grid_wait();
+  grid_release();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= g.ng) return;
   const int x = (int)(i % g.nx), y = (int)((i / g.nx) % g.ny), z = (int)(i / g.sz);
@@ -1705,6 +1726,8 @@ __global__ void k_phase_source(Geom g, PhaseArrays a, Ctrl* ctrl, double mult) {
 // set_ghost_cells as gather (values before the sweep) + scatter
 __global__ void k_ghost_gather(int nghost, const int32_t* src, const uint8_t* sgn,
                                const double* cons, long long n, double* tmp) {
+  grid_wait();
+  grid_release();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nghost) return;
   const long long s = src[k];
@@ -1717,6 +1740,8 @@ __global__ void k_ghost_gather(int nghost, const int32_t* src, const uint8_t* sg
 }
 __global__ void k_ghost_scatter(int nghost, const int32_t* dst, const double* tmp, double* cons,
                                 long long n) {
+  grid_wait();
+  grid_release();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nghost) return;
   const long long d = dst[k];
@@ -1965,6 +1990,8 @@ __global__ void k_phase_faces(Geom g, PhaseArrays a, double* F) {
 // and floors (flux.f90:186-230), from cons to out
 __global__ void k_phase_ghost_update(int nghost, const int32_t* dst, Geom g, const double* cons,
                                      const double* cons_old, double* out, Ctrl* ctrl, int avg) {
+  grid_wait();
+  grid_release();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= nghost) return;
   const long long i = dst[j], n = g.ng;
@@ -2117,20 +2144,16 @@ __global__ void k_soa_to_aos(const double* soa, double* aos, long long n, int k)
 }  // namespace
 
 cudaError_t phase_state(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream_t s) {
-  k_phase_state<<<nblk(g.ng), PB, 0, s>>>(g, a, ctrl);
-  return cudaGetLastError();
+  return launch_after(true, k_phase_state, nblk(g.ng), PB, 0, s, g, a, ctrl);
 }
 cudaError_t phase_velocity(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream_t s) {
-  k_phase_velocity<<<nblk(g.ng), PB, 0, s>>>(g, a, ctrl);
-  return cudaGetLastError();
+  return launch_after(true, k_phase_velocity, nblk(g.ng), PB, 0, s, g, a, ctrl);
 }
 cudaError_t phase_state_velocity(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream_t s) {
-  k_phase_state_velocity<<<nblk(g.ng), PB, 0, s>>>(g, a, ctrl);
-  return cudaGetLastError();
+  return launch_after(true, k_phase_state_velocity, nblk(g.ng), PB, 0, s, g, a, ctrl);
 }
 cudaError_t phase_courant(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream_t s) {
-  k_phase_courant<<<nblk(g.ng), PB, 0, s>>>(g, a, ctrl);
-  return cudaGetLastError();
+  return launch_after(true, k_phase_courant, nblk(g.ng), PB, 0, s, g, a, ctrl);
 }
 cudaError_t phase_avisc(const Geom& g, const double* u, const double avmag[3], double* qq,
                         cudaStream_t s) {
@@ -2168,23 +2191,23 @@ cudaError_t phase_calc_gforce(const Geom& g, const double* phi, double* gforce, 
 }
 
 cudaError_t phase_source(const Geom& g, PhaseArrays& a, Ctrl* ctrl, double mult, cudaStream_t s) {
-  k_phase_source<<<nblk(g.ng), PB, 0, s>>>(g, a, ctrl, mult);
-  return cudaGetLastError();
+  return launch_after(true, k_phase_source, nblk(g.ng), PB, 0, s, g, a, ctrl, mult);
 }
 cudaError_t phase_ghost(int nghost, const int32_t* dst, const int32_t* src, const uint8_t* sgn,
                         PhaseArrays& a, long long ng, cudaStream_t s) {
   if (nghost <= 0) return cudaSuccess;
-  k_ghost_gather<<<nblk(nghost), PB, 0, s>>>(nghost, src, sgn, a.cons, ng, a.gtmp);
-  k_ghost_scatter<<<nblk(nghost), PB, 0, s>>>(nghost, dst, a.gtmp, a.cons, ng);
-  return cudaGetLastError();
+  const cudaError_t e = launch_after(true, k_ghost_gather, nblk(nghost), PB, 0, s, nghost, src, sgn,
+                                     a.cons, ng, a.gtmp);
+  if (e != cudaSuccess) return e;
+  return launch_after(true, k_ghost_scatter, nblk(nghost), PB, 0, s, nghost, dst,
+                      a.gtmp, a.cons, ng);
 }
 template <int AVG, int PM, bool THREED>
 static cudaError_t launch_phase_tile(const StageArgs& t, int ntiles, cudaStream_t s) {
   const size_t smem = Shape0::SMEM_DOUBLES * sizeof(double);
   const cudaError_t e = ensure_dyn_smem((const void*)k_phase_tile<AVG, PM, THREED>, smem);
   if (e != cudaSuccess) return e;
-  k_phase_tile<AVG, PM, THREED><<<ntiles, Shape0::NT, smem, s>>>(t);
-  return cudaGetLastError();
+  return launch_after(true, k_phase_tile<AVG, PM, THREED>, ntiles, Shape0::NT, smem, s, t);
 }
 template <int AVG>
 static cudaError_t launch_phase_tile(const Geom& g, const StageArgs& t, int ntiles,
@@ -2214,15 +2237,15 @@ cudaError_t phase_flux(const Geom& g, PhaseArrays& a, Ctrl* ctrl, int avg, cudaS
     t.geom = a.geom;
     t.tiles = a.tiles;
     t.ncells_total = g.ng;
-    const cudaError_t e = avg ? launch_phase_tile<1>(g, t, a.ntiles, s)
-                              : launch_phase_tile<0>(g, t, a.ntiles, s);
+    cudaError_t e = avg ? launch_phase_tile<1>(g, t, a.ntiles, s)
+                        : launch_phase_tile<0>(g, t, a.ntiles, s);
+    if (e == cudaSuccess && a.nghost > 0)
+      e = launch_after(true, k_phase_ghost_update, nblk(a.nghost), PB, 0, s, a.nghost, a.gdst, g,
+                       a.cons, a.cons_old, a.states, ctrl, avg);
     if (e != cudaSuccess) return e;
-    if (a.nghost > 0)
-      k_phase_ghost_update<<<nblk(a.nghost), PB, 0, s>>>(a.nghost, a.gdst, g, a.cons, a.cons_old,
-                                                         a.states, ctrl, avg);
     std::swap(a.cons, a.states);                    // states: the cons before the flux
     if (save_old) std::swap(a.cons_old, a.states);
-    return cudaGetLastError();
+    return cudaSuccess;
   }
   if (save_old) {
     const cudaError_t e = phase_copy_old(g, a, s);

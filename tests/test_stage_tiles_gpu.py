@@ -65,3 +65,25 @@ def test_tile_edges_per_phase(n, walls, dx):
     assert g.status()[1] == 0
     o.close()
     g.close()
+
+
+@pytest.mark.parametrize("phase_only", [False, True])
+@pytest.mark.parametrize("n", [(8, 1, 1), (32, 32, 32), (75, 61, 47)])
+def test_dependent_launches(n, phase_only):
+    """Launches that start before the one ahead of them is through (a run's, and single
+    steps') against launches with events between them, and the oracle."""
+    nz = n[2] + 4 if n[2] > 1 else 1
+    st = small_random_box(nx=n[0] + 4, ny=n[1] + 4, nz=nz, seed=7)
+    o, g = make_pair(st, phase_only=phase_only)
+    step_both(o, g, 12)
+    other = make_pair(st, phase_only=phase_only)
+    timed = other[1]
+    for k in range(12):
+        timed.profile(k % 2 == 0)
+        timed.step()
+    run = make_pair(st, phase_only=phase_only)
+    run[1].run(nsteps=12)
+    want = g.download()[0]
+    assert np.array_equal(want, timed.download()[0]) and np.array_equal(want, run[1].download()[0])
+    for x in (o, g, *other, *run):
+        x.close()
