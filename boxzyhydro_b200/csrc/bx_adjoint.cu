@@ -34,6 +34,7 @@
 #include "bx_adjoint_math.cuh"
 #include "bx_handle.h"
 #include "bx_internal.h"
+#include "bx_launch.cuh"
 
 using namespace bx;
 
@@ -90,6 +91,8 @@ __device__ __forceinline__ void decode(const Geom& g, long long i, int& x, int& 
 // P planes: 0 rho, 1-3 u, 4 p, 5 eps, 6 c
 // grid: x threads by (y, z) blocks
 __global__ void k_r1_prims(Geom g, int stage, const double* A, const double* B, double* P) {
+  grid_wait();
+  grid_release();
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
   if (x >= g.nx) return;
   const long long i = x + (long long)y * g.sy + (long long)z * g.sz;
@@ -254,6 +257,8 @@ template <int DIR, bool POW2>
 __global__ void __launch_bounds__(DIR == 0 ? 128 : 256, DIR == 0 ? 4 : 2)
 k_rdir(Geom g, const double* P, const double* lamL, double lscale, double dt, double* PA,
        RShape sh) {
+  grid_wait();
+  grid_release();
   const int NL = sh.NL, W = sh.W, NQ = W + 6, NS = W + 4, NF = W + 3, ND = W + 2;
   using M = RMem<DIR>;
   constexpr int T = M::T;  // plane stride of the states, faces and MUSCL cells
@@ -534,6 +539,8 @@ template <int STAGE>
 __global__ void k_rcell(Geom g, const double* SA, const double* SB, const double* P,
                         const double* PA, const double* lin, double* o1, double* o2,
                         const double* X, int nsrc, int nbx, unsigned nedge) {
+  grid_wait();
+  grid_release();
   // the first nedge blocks take the two x-edge columns, whose cells all fold
   // ghosts (their long chains start first); the others, nbx blocks a row, the
   // columns between them, where a warp takes the ghost path together or not at
@@ -563,19 +570,19 @@ __global__ void k_rcell(Geom g, const double* SA, const double* SB, const double
   double gq[7], a[10], gA[5], gB[5], li[5], xs[5];
   CvIn v;
 #pragma unroll
-  for (int q = 0; q < 7; ++q) gq[q] = __ldg(PA + q * n + i);
-  v.rho = __ldg(P + i);
-  v.u[0] = __ldg(P + n + i); v.u[1] = __ldg(P + 2 * n + i); v.u[2] = __ldg(P + 3 * n + i);
-  v.p = __ldg(P + 4 * n + i); v.e = __ldg(P + 5 * n + i); v.cs = __ldg(P + 6 * n + i);
+  for (int q = 0; q < 7; ++q) gq[q] = __ldca(PA + q * n + i);
+  v.rho = __ldca(P + i);
+  v.u[0] = __ldca(P + n + i); v.u[1] = __ldca(P + 2 * n + i); v.u[2] = __ldca(P + 3 * n + i);
+  v.p = __ldca(P + 4 * n + i); v.e = __ldca(P + 5 * n + i); v.cs = __ldca(P + 6 * n + i);
   v.aE = 0.0; v.bd = 1.0; v.bm[0] = v.bm[1] = v.bm[2] = 0.0;
   if (STAGE == 1) {
-    v.aE = __ldg(SA + 4 * n + i);
-    v.bd = __ldg(SB + i);
-    v.bm[0] = __ldg(SB + n + i); v.bm[1] = __ldg(SB + 2 * n + i); v.bm[2] = __ldg(SB + 3 * n + i);
+    v.aE = __ldca(SA + 4 * n + i);
+    v.bd = __ldca(SB + i);
+    v.bm[0] = __ldca(SB + n + i); v.bm[1] = __ldca(SB + 2 * n + i); v.bm[2] = __ldca(SB + 3 * n + i);
   }
-  for (int q = 0; q < 5; ++q) li[q] = __ldg(lin + q * n + i);
+  for (int q = 0; q < 5; ++q) li[q] = __ldca(lin + q * n + i);
   if (STAGE == 0 && nsrc > 0)
-    for (int q = 0; q < 5; ++q) xs[q] = __ldg(X + q * n + i);
+    for (int q = 0; q < 5; ++q) xs[q] = __ldca(X + q * n + i);
   cons_vjp_v(g, STAGE, v, gq, gA, gB);
   for (int q = 0; q < 5; ++q) { a[q] = gA[q]; a[5 + q] = gB[q]; }
   const bool edge = x == g.ax0 || x == g.ax1 - 1 || y == g.ay0 || y == g.ay1 - 1 ||
@@ -597,7 +604,7 @@ __global__ void k_rcell(Geom g, const double* SA, const double* SB, const double
       CvIn w = v;
       double hq[7];
 #pragma unroll
-      for (int q = 0; q < 7; ++q) hq[q] = __ldg(PA + q * n + gi);
+      for (int q = 0; q < 7; ++q) hq[q] = __ldca(PA + q * n + gi);
 #pragma unroll
       for (int q = 0; q < 3; ++q)
         if (flip && q == dir) {
@@ -690,6 +697,8 @@ __global__ void k_adj_src_vjp(Geom g, const double* X, int nsrc, double* lam) {
 }
 
 __global__ void k_set_clock(Ctrl* c, double dt, int active) {
+  grid_wait();
+  grid_release();
   c->dt = dt;
   c->active = active;
 }
@@ -1159,7 +1168,7 @@ static int fwd_step(bx_adj* A, const double* X, int nsrc, double dt, double* Y,
   a.nsrc = nsrc;
   a.after = 1;
   a.U = A->P;  // the primitives are rebuilt by every reverse stage
-  k_set_clock<<<1, 1, 0, h->stream>>>(h->d_ctrl, dt, 1);
+  ACK(launch_after(true, k_set_clock, 1, 1, 0, h->stream, h->d_ctrl, dt, 1));
   a.X = X;
   a.Y = nullptr;
   a.out = c1out ? c1out : A->W1;
@@ -1186,8 +1195,11 @@ static cudaError_t launch_rdir(const Geom& g, const double* P, const double* lam
   if (e != cudaSuccess) return e;
   const long long ngrp = (nlines + sh.NL - 1) / sh.NL;
   const dim3 grid((unsigned)(ngrp * sh.nseg));
-  k_rdir<DIR, POW2><<<grid, sh.threads, RMem<DIR>::bytes, s>>>(g, P, lamL, lscale, dt, PA, sh);
-  return cudaGetLastError();
+  // The next direction's blocks start in the last wave's gaps on small grids (16 steps
+  // of 64^3: 435 -> 423 us per step, 48^3 259 -> 248); on larger ones they take the
+  // slots and the L1 of blocks still at work (80^3 818 -> 847, 96^3 1269 -> 1342).
+  return launch_after(g.ng < (1 << 19), k_rdir<DIR, POW2>, grid, sh.threads, RMem<DIR>::bytes, s, g, P, lamL,
+                      lscale, dt, PA, sh);
 }
 
 template <int DIR>
@@ -1208,7 +1220,7 @@ static int rev_stage(bx_adj* A, int stage, const double* SA, const double* SB, c
   // primitives of every cell: one block row per (y, z)
   const int tp = std::min(512, ((g.nx + 31) / 32) * 32);
   const dim3 pgrid((unsigned)((g.nx + tp - 1) / tp), (unsigned)g.ny, (unsigned)g.nz);
-  k_r1_prims<<<pgrid, tp, 0, s>>>(g, stage, SA, SB, A->P);
+  ACK(launch_after(true, k_r1_prims, pgrid, tp, 0, s, g, stage, SA, SB, A->P));
   // interior cells
   const int nxm = std::max(1, g.ax1 - g.ax0 - 2), tc = std::min(256, ((nxm + 31) / 32) * 32);
   const int nbx = (nxm + tc - 1) / tc;
@@ -1218,11 +1230,9 @@ static int rev_stage(bx_adj* A, int stage, const double* SA, const double* SB, c
   ACK(launch_rdir<0>(g, A->P, lamL, lscale, dt, A->PA, s));
   ACK(launch_rdir<1>(g, A->P, lamL, lscale, dt, A->PA, s));
   if (g.threed) ACK(launch_rdir<2>(g, A->P, lamL, lscale, dt, A->PA, s));
-  if (stage == 1)
-    k_rcell<1><<<cgrid, tc, 0, s>>>(g, SA, SB, A->P, A->PA, lin, o1, o2, X, nsrc, nbx, nedge);
-  else
-    k_rcell<0><<<cgrid, tc, 0, s>>>(g, SA, SB, A->P, A->PA, lin, o1, o2, X, nsrc, nbx, nedge);
-  ACK(cudaGetLastError());
+  // (an ordinary launch: started early it is slower at 64^3, 428 against 423 us a step)
+  ACK(launch_after(false, stage == 1 ? k_rcell<1> : k_rcell<0>, cgrid, tc, 0, s, g, SA, SB, A->P,
+                   A->PA, lin, o1, o2, X, nsrc, nbx, nedge));
   return BX_OK;
 }
 
