@@ -262,7 +262,7 @@ int bx_batch_get_clock(bx_batch *b, int32_t box, double *time, double *dt, doubl
                        int64_t *step);
 /* nsteps iterations of every box's main loop (boxes at endtime stop).  use_graph != 0:
  * the run is captured once into a CUDA graph and replayed.  The launches are three per
- * step (dt, stage 0, stage 1, clock), or, in persistent mode (bx_batch_set_persistent,
+ * step (stage 0, stage 1, clock), or, in persistent mode (bx_batch_set_persistent,
  * or chosen by bx_batch_autotune), one launch for the whole run after the first
  * step's dt: its blocks take (step, stage, tile) items from a queue in step order and
  * wait for what an item reads (a stage-0 tile for its box's dt, a stage-1 tile for
