@@ -213,6 +213,14 @@ static int create_handle(const bx_params* params, bx_handle** out, bool lean) {
   return BX_OK;
 }
 
+// the cached graphs of bx_run (none of them in flight)
+static void drop_run_graphs(bx_handle* h) {
+  for (cudaGraphExec_t& x : h->run_graph) {
+    if (x) cudaGraphExecDestroy(x);
+    x = nullptr;
+  }
+}
+
 extern "C" {
 
 int bx_destroy(bx_handle* h) {
@@ -229,8 +237,7 @@ int bx_destroy(bx_handle* h) {
   cudaFree(h->pa.gtmp);
   cudaFree(h->pa.muc);
   cudaFree(h->d_eos);
-  for (cudaGraphExec_t x : h->run_graph)
-    if (x) cudaGraphExecDestroy(x);
+  drop_run_graphs(h);
   for (cudaStream_t x : h->hs)
     if (x) cudaStreamDestroy(x);
   for (cudaEvent_t e : h->hev) cudaEventDestroy(e);
@@ -612,14 +619,40 @@ int bx_set_eos_table(bx_handle* h, const bx_eos_table* t) {
     p[5] = other ? 1.0 / (t->rho_table[rp] - t->rho_table[r]) : 0.0;
     p[6] = other ? 1.0 : 0.0;
   }
+  // whatever is queued reads the tables in place; the run graphs hold their
+  // addresses and extents, so they go with them
+  CK(cudaStreamSynchronize(h->stream));
+  drop_run_graphs(h);
   cudaFree(h->d_eos);
   h->d_eos = nullptr;
-  CK(dalloc((void**)&h->d_eos, host.size() * sizeof(double)));
-  CK(cudaMemcpy(h->d_eos, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice));
-  if (!h->pa.muc) {
-    CK(dalloc((void**)&h->pa.muc, h->g.ng * sizeof(double)));
-    CK(cudaMemset(h->pa.muc, 0, h->g.ng * sizeof(double)));
+  // on failure the handle is one without tables: no step runs until they are set
+  auto fail = [&](cudaError_t e, const char* what) {
+    cudaGetLastError();
+    cudaFree(h->d_eos);
+    cudaFree(h->pa.muc);
+    h->d_eos = h->pa.muc = nullptr;
+    h->pa.eos = EosDev{};
+    update_eligible(h);
+    return set_err(h, BX_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+  };
+  const size_t bytes = host.size() * sizeof(double), mucb = h->g.ng * sizeof(double);
+  if (const cudaError_t e = dalloc((void**)&h->d_eos, bytes)) {
+    h->d_eos = nullptr;
+    return fail(e, "memory for the EOS tables");
   }
+  cudaError_t ce =
+      cudaMemcpyAsync(h->d_eos, host.data(), bytes, cudaMemcpyHostToDevice, h->stream);
+  if (!h->pa.muc) {
+    const cudaError_t e = dalloc((void**)&h->pa.muc, mucb);
+    if (e != cudaSuccess) {
+      h->pa.muc = nullptr;
+      return fail(e, "memory for muc_array");
+    }
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(h->pa.muc, 0, mucb, h->stream);
+  }
+  if (ce == cudaSuccess) ce = eos_log_rows(h->d_eos + 8 * n2, (int)nr, h->stream);
+  if (ce == cudaSuccess) ce = cudaStreamSynchronize(h->stream);
+  if (ce != cudaSuccess) return fail(ce, "copying the EOS tables");
   EosDev& e = h->pa.eos;
   e.neos = t->neos;
   e.neos_rho = t->neos_rho;
@@ -629,8 +662,6 @@ int bx_set_eos_table(bx_handle* h, const bx_eos_table* t) {
   e.tk_bgrnd = t->tk_bgrnd;
   e.pack = h->d_eos;
   e.rows = h->d_eos + 8 * n2;
-  CK(eos_log_rows(h->d_eos + 8 * n2, (int)nr, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
   // the fused kernels read the tables from here on (not while a force is set)
   update_eligible(h);
   return BX_OK;

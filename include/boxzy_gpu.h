@@ -157,7 +157,9 @@ int bx_read_celldump(bx_handle *h, const char *path, double *phi, double *time, 
  * gamma, mu and T from them by get_gamma2 (eos.f90:653-699) as state.f90:60-79
  * does (including the disk scale-height branch for nz == 1).  Such grids run the
  * fused stage kernels (nz != 1, no force) or the per-phase kernels;
- * bx_set_eos_table must come before the first step. */
+ * bx_set_eos_table must come before the first step.  It may be called again with
+ * other tables, of other extents too; where it fails for want of memory the handle is
+ * left without tables and its steps are refused until a call succeeds. */
 typedef struct bx_eos_table {
   int32_t neos;            /* NEOS = NEOS_T: entries per density (eng_table2 rows) */
   int32_t neos_rho;        /* NEOS_RHO */
