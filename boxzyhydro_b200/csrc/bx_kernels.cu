@@ -683,8 +683,8 @@ __device__ __forceinline__ void ctrl_store_cg(Ctrl* p, const Ctrl& c) {
 enum : unsigned { kItemY = 1u << 12, kItemGhost = 1u << 13, kItemIn = 1u << 14 };
 
 // PH: the flux of the per-phase path (flux.f90:6-230) on the reference's arrays:
-// u and p are read, not derived, ghost cells are cells like any other, and nothing of
-// the sources, guards or the next step's rate is done here (phase_flux).
+// u and p are read, not derived, a ghost's values are its own, not its donor's, and
+// nothing of the sources, guards or the next step's rate is done here (phase_flux).
 template <class S, int STAGE, bool POW2, bool THREED, bool GRAV, bool CG = false, bool PH = false>
 __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, const Geom& g,
                                            Ctrl* C, double dt, int nsrc, double* sm,
@@ -758,9 +758,11 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
       in = j < 4 && cx < w;
     }
     if (in) {
-      Place p{g.base + bx0 + cx + (long long)(by0 + cy) * g.sy + (long long)g.az0 * g.sz,
-              false, false, false};
-      if (!PH) p = place_of(g, bx0 + cx, by0 + cy, g.az0);
+      // (PH: own_place)
+      const int hx = PH ? min(max(bx0 + cx, g.ax0 - 1), g.ax1) : bx0 + cx;
+      const int hy = PH ? min(max(by0 + cy, g.ay0 - 1), g.ay1) : by0 + cy;
+      Place p{g.base + hx + (long long)hy * g.sy + (long long)g.az0 * g.sz, false, false, false};
+      if (!PH) p = place_of(g, hx, hy, g.az0);
       hpc = p.c - (long long)g.az0 * g.sz;
       // (a halo cell of the x/y halo is beyond one wall at most)
       hc = ((cy + 2) * PW + cx + 2) | (p.fx ? 1 << 12 : 0) | (p.fy ? 1 << 13 : 0);
@@ -768,9 +770,14 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
   }
   const long long co = g.base + gx + (long long)gy * g.sy;  // the own column
   auto zs = [&](int k) -> double& { return ZS[k * NOWN + tid]; };
+  // PH: the outer ghost layer reads as the inner one.  Only the inner one's slopes take
+  // it, which are zero whatever the arrays hold there (flux.f90:53-57; their factor in
+  // muscl_states is zero, but a caller's NaN times zero is not)
   auto own_place = [&](int z) {
     Place p{0, false, false, false};
-    const int zz = THREED && !PH ? remap_axis(z, g.az0, g.az1, g.wall[4], g.wall[5], p.fz) : z;
+    int zz = z;
+    if (THREED) zz = PH ? min(max(z, g.az0 - 1), g.az1)
+                        : remap_axis(z, g.az0, g.az1, g.wall[4], g.wall[5], p.fz);
     p.c = co + (long long)zz * g.sz;
     return p;
   };
