@@ -201,6 +201,7 @@ static int create_handle(const bx_params* params, bx_handle** out, bool lean) {
   h->pa.ntiles = h->ntiles;
   h->pa.nghost = h->nghost;
   h->pa.gdst = h->d_dst;
+  h->pa.after = 1;
   CKC(dalloc((void**)&h->d_ctrl, sizeof(Ctrl)));
   CKC(cudaMallocHost((void**)&h->h_ctrl, sizeof(Ctrl)));
   std::memset(&h->clock, 0, sizeof(Ctrl));
@@ -721,7 +722,7 @@ static int phase_step(bx_handle* h) {
   CK(phase_state(g, a, c, s));
   CK(cudaMemsetAsync(&c->rate_bits, 0, sizeof(unsigned long long), s));
   CK(phase_courant(g, a, c, s));
-  CK(launch_dt(c, 1, s, true));
+  CK(launch_dt(c, 1, s, a.after));
   CK(phase_source(g, a, c, 0.5, s));   // source(time,0) with dt/2
   if (int r = ghost2(h)) return r;
   CK(phase_state_velocity(g, a, c, s));
@@ -734,7 +735,7 @@ static int phase_step(bx_handle* h) {
   CK(phase_source(g, a, c, 0.5, s));   // source(time+dt,1) with dt/2
   if (int r = ghost2(h)) return r;
   CK(phase_state_velocity(g, a, c, s));
-  CK(launch_end(c, 1, s, true));
+  CK(launch_end(c, 1, s, a.after));
   h->launches += 22 + (g.ang || g.tab ? 3 : 0);
   return BX_OK;
 }
@@ -1170,6 +1171,7 @@ int bx_profile(bx_handle* h, int32_t enable) {
   if (enable && !h->ev[0])
     for (int k = 0; k < 3; ++k) CK(cudaEventCreate(&h->ev[k]));
   h->prof = enable != 0;
+  h->pa.after = !h->prof;  // as fused_launch
   h->ms_stage[0] = h->ms_stage[1] = 0.0;
   h->n_stage = 0;
   h->launches = 0;

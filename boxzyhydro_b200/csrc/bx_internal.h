@@ -237,6 +237,7 @@ struct PhaseArrays {
   int ntiles;
   int nghost;       // the ghost cells, in index order
   const int32_t* gdst;
+  int after;        // the launches may start before the stream's last kernel is through
 };
 
 cudaError_t phase_state(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream_t s);

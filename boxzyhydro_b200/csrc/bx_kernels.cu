@@ -2151,16 +2151,16 @@ __global__ void k_soa_to_aos(const double* soa, double* aos, long long n, int k)
 }  // namespace
 
 cudaError_t phase_state(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream_t s) {
-  return launch_after(true, k_phase_state, nblk(g.ng), PB, 0, s, g, a, ctrl);
+  return launch_after(a.after, k_phase_state, nblk(g.ng), PB, 0, s, g, a, ctrl);
 }
 cudaError_t phase_velocity(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream_t s) {
-  return launch_after(true, k_phase_velocity, nblk(g.ng), PB, 0, s, g, a, ctrl);
+  return launch_after(a.after, k_phase_velocity, nblk(g.ng), PB, 0, s, g, a, ctrl);
 }
 cudaError_t phase_state_velocity(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream_t s) {
-  return launch_after(true, k_phase_state_velocity, nblk(g.ng), PB, 0, s, g, a, ctrl);
+  return launch_after(a.after, k_phase_state_velocity, nblk(g.ng), PB, 0, s, g, a, ctrl);
 }
 cudaError_t phase_courant(const Geom& g, PhaseArrays& a, Ctrl* ctrl, cudaStream_t s) {
-  return launch_after(true, k_phase_courant, nblk(g.ng), PB, 0, s, g, a, ctrl);
+  return launch_after(a.after, k_phase_courant, nblk(g.ng), PB, 0, s, g, a, ctrl);
 }
 cudaError_t phase_avisc(const Geom& g, const double* u, const double avmag[3], double* qq,
                         cudaStream_t s) {
@@ -2198,15 +2198,15 @@ cudaError_t phase_calc_gforce(const Geom& g, const double* phi, double* gforce, 
 }
 
 cudaError_t phase_source(const Geom& g, PhaseArrays& a, Ctrl* ctrl, double mult, cudaStream_t s) {
-  return launch_after(true, k_phase_source, nblk(g.ng), PB, 0, s, g, a, ctrl, mult);
+  return launch_after(a.after, k_phase_source, nblk(g.ng), PB, 0, s, g, a, ctrl, mult);
 }
 cudaError_t phase_ghost(int nghost, const int32_t* dst, const int32_t* src, const uint8_t* sgn,
                         PhaseArrays& a, long long ng, cudaStream_t s) {
   if (nghost <= 0) return cudaSuccess;
-  const cudaError_t e = launch_after(true, k_ghost_gather, nblk(nghost), PB, 0, s, nghost, src, sgn,
+  const cudaError_t e = launch_after(a.after, k_ghost_gather, nblk(nghost), PB, 0, s, nghost, src, sgn,
                                      a.cons, ng, a.gtmp);
   if (e != cudaSuccess) return e;
-  return launch_after(true, k_ghost_scatter, nblk(nghost), PB, 0, s, nghost, dst,
+  return launch_after(a.after, k_ghost_scatter, nblk(nghost), PB, 0, s, nghost, dst,
                       a.gtmp, a.cons, ng);
 }
 template <int AVG, int PM, bool THREED>
@@ -2214,7 +2214,7 @@ static cudaError_t launch_phase_tile(const StageArgs& t, int ntiles, cudaStream_
   const size_t smem = Shape0::SMEM_DOUBLES * sizeof(double);
   const cudaError_t e = ensure_dyn_smem((const void*)k_phase_tile<AVG, PM, THREED>, smem);
   if (e != cudaSuccess) return e;
-  return launch_after(true, k_phase_tile<AVG, PM, THREED>, ntiles, Shape0::NT, smem, s, t);
+  return launch_after(t.after, k_phase_tile<AVG, PM, THREED>, ntiles, Shape0::NT, smem, s, t);
 }
 template <int AVG>
 static cudaError_t launch_phase_tile(const Geom& g, const StageArgs& t, int ntiles,
@@ -2244,10 +2244,11 @@ cudaError_t phase_flux(const Geom& g, PhaseArrays& a, Ctrl* ctrl, int avg, cudaS
     t.geom = a.geom;
     t.tiles = a.tiles;
     t.ncells_total = g.ng;
+    t.after = a.after;
     cudaError_t e = avg ? launch_phase_tile<1>(g, t, a.ntiles, s)
                         : launch_phase_tile<0>(g, t, a.ntiles, s);
     if (e == cudaSuccess && a.nghost > 0)
-      e = launch_after(true, k_phase_ghost_update, nblk(a.nghost), PB, 0, s, a.nghost, a.gdst, g,
+      e = launch_after(a.after, k_phase_ghost_update, nblk(a.nghost), PB, 0, s, a.nghost, a.gdst, g,
                        a.cons, a.cons_old, a.states, ctrl, avg);
     if (e != cudaSuccess) return e;
     std::swap(a.cons, a.states);                    // states: the cons before the flux

@@ -218,7 +218,8 @@ int bx_status(bx_handle *h, uint32_t *status_bits, int32_t *last_path);
  * zero-copy users; valid until the next call on the handle. */
 int bx_device_cons(bx_handle *h, double **cons_soa, int64_t *ngrid);
 
-/* Timing hooks: with profiling on, every fused step records CUDA events around
+/* Timing hooks: with profiling on, no kernel of a step starts before the one ahead of
+ * it is through, and every fused step records CUDA events around
  * its two stage kernels on the handle's stream; bx_profile_read returns the
  * accumulated stage times (ms), the number of fused steps timed and the number
  * of this library's kernels launched since bx_profile was called. */
