@@ -107,7 +107,9 @@ int bx_upload_conserved(bx_handle *h, const double *cons);
  * Any pointer may be NULL. */
 int bx_download(bx_handle *h, double *cons, double *u, double *p);
 
-/* The main-loop clock of main.f90:102,196-199: time, dtold and step. */
+/* The main-loop clock of main.f90:102,196-199: time, dtold and step.  bx_get_clock
+ * gives the host's copy, current after every call that moves the clock; it does not
+ * wait for the stream. */
 int bx_set_clock(bx_handle *h, double time, double dtold, int64_t step);
 int bx_get_clock(bx_handle *h, double *time, double *dt, double *dtold, int64_t *step);
 
@@ -205,7 +207,10 @@ int bx_set_gforce(bx_handle *h, const double *gforce);
 /* The gravity coupling of a run with a potential solver (main.f90:143-149,477-483
  * under USEPOTENTIAL): phi(ngrid) from the host's solver, turned into gforce on the
  * device by calc_gforce (utils.f90:549-571, central differences on interior cells).
- * Call it whenever the solver updates phi (each step); NULL removes the force.
+ * Call it whenever the solver updates phi (each step); NULL removes the force.  On
+ * return phi has been read and may be reused; the force is formed in stream order,
+ * before whatever the handle does next, and an error of its kernel is reported by the
+ * next call that waits for the stream.
  * Both sources of the next step apply the force; grids the fused path takes run
  * it in the stage kernels. */
 int bx_set_phi(bx_handle *h, const double *phi);
