@@ -407,7 +407,7 @@ def batched_measure(args, rank, world, local, init_dist=True):
             tuned.append({"tile_depth": "whole box" if zc >= 1 << 30 else
                           ("default rule" if zc == 0 else zc), "trial_ms_per_step": tms,
                           "tile_columns": f"{ttx}x{tty}",
-                          "launch_form": "persistent" if b.persistent else "4 per step"})
+                          "launch_form": "persistent" if b.persistent else "3 per step"})
         b.run(args.steps)
         inf = b.info()
         total_ms += inf["last_run_ms"]

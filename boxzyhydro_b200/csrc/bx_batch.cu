@@ -119,18 +119,12 @@ int bx_batch_destroy(bx_batch* b);
 
 const char* bx_batch_last_error(bx_batch* b) { return b ? b->err.c_str() : g_batch_err.c_str(); }
 
-// Tiles of every box, longest first.  zc: the z extent of a column tile
-// (interior planes; capped at each box's depth), or 0 for the default rule: a
-// tile marches through the whole box depth when the ensemble has enough
-// columns to fill the GPU many times over (no z warm-up repeated per chunk),
-// else the depth of at most 32 planes whose tiles, longest first on the resident
-// blocks, are through soonest (default_depth).
 // The planes of a tile for which the list of an ensemble that does not fill the GPU
 // many times over ends first: a tile costs its planes and about one more (the two
 // warm-up rounds of its z pipeline), and goes to the block that is free first.  With
 // a fixed 32 planes a dozen boxes leave most blocks idle behind the deepest tiles:
-// 12 boxes of 32 to 64 cells a side 602 us per step against 493 with 8 planes, 4 of 16
-// to 40 452 against 124 with 5, 8 of 20 to 30 429 against 89 with 3.
+// 12 boxes of 32 to 64 cells a side 604 us per step against 488 with this rule, 4 of 16
+// to 40 441 against 118, 8 of 20 to 30 411 against 82, 16 of 40 to 64 1044 against 790.
 static int default_depth(const bx_batch* b, int TX, int TY, long long slots) {
   int best = 32;
   double best_t = 1e300;
@@ -168,6 +162,12 @@ static int default_depth(const bx_batch* b, int TX, int TY, long long slots) {
   return best;
 }
 
+// Tiles of every box, longest first.  zc_req: the z extent of a column tile
+// (interior planes; capped at each box's depth), or 0 for the default rule: a
+// tile marches through the whole box depth when the ensemble has enough
+// columns to fill the GPU many times over (no z warm-up repeated per chunk),
+// else the depth of at most 32 planes whose tiles, longest first on the resident
+// blocks, are through soonest (default_depth).
 static std::vector<Tile> batch_tiles(const bx_batch* b, int zc_req, int shape) {
   const int TX = shape_tx(shape), TY = shape_ty(shape);
   int dev = 0, sms = 148;

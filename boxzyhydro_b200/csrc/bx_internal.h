@@ -99,7 +99,7 @@ struct TileShape {
   static constexpr int NP = (TY + 4) * PW;   // prim plane cells
   static constexpr int NSX = TY * (TX + 2);  // x-state cells
   static constexpr int NSY = (TY + 2) * TX;  // y-state cells
-    // per-column z-pipeline slots (3-D): the z flux below the own cell and its
+  // per-column z-pipeline slots (3-D): the z flux below the own cell and its
   // difference over the cell (5 + 5) and the plus z-state carried to the next
   // plane (NSF), kept in shared memory so the x/y phases have the registers
   static constexpr int NZS = 10 + NSF;
@@ -112,7 +112,8 @@ using Shape1 = TileShape<16, 16>;
 // the tabulated EOS and angular-momentum fluxing (single grids only): 32 x 6
 // columns, so the larger primitive and face-state sets still fit two blocks per
 // SM, and a thread per column: with 192 threads a thread may hold 168 registers and
-// nothing spills (with 256 threads, 128 registers: 172 bytes per thread with
+// of the eight 3-D instances only flux_ang's stage 1 with spacings no power of two
+// spills (40 bytes; with 256 threads, 128 registers: 172 bytes per thread with
 // flux_ang, 76 with the tables; measured 569 against 501 us and 629 against 611
 // per 96^3 step; 224 threads get the same 128 registers)
 using Shape2 = TileShape<32, 6, 1, 192>;
@@ -120,7 +121,8 @@ using Shape3 = TileShape<32, 6, 2, 192>;
 // grids of at most one tile per SM, where a second block per SM has nothing to do:
 // twice the threads on a tile, so those without a column take the halo's primitives
 // and the rim's states and faces beside the columns' own (two rounds instead of
-// three; 32^3 28.4 against 26.6 us per step, 512-cell tube 15.6 against 14.3; beyond
+// three; 512-cell tube 13.2 against 11.9 us per step, an upload and 32 steps of 32^3
+// 1037 against 979, the stepped 4x196 tube even; beyond
 // one tile per SM two 256-thread blocks hide each other's barriers);
 // kWideShape's extents are shape 0's
 using Shape4 = TileShape<32, 8, 0, 512>;

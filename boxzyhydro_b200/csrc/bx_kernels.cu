@@ -659,10 +659,10 @@ __device__ __forceinline__ void ctrl_store_cg(Ctrl* p, const Ctrl& c) {
 // fluxes go where the states they came from were, so nothing of D is overwritten
 // by A of the next plane.
 //
-// What bounds it (ncu, 128^3): not memory (DRAM 8-12 % busy) but the latency of
-// the FP64 chains at 16 warps per SM, the registers' limit: 53 % of issue slots
-// and 45 % of the FP64 pipe; of 7.1 warp cycles per instruction 1.65 wait on a
-// fixed latency, 1.2 at a barrier, 0.5 for the FP64 pipe, 0.6-0.8 for global
+// What bounds it (ncu, 128^3): not memory (DRAM 10-15 % busy) but the latency of
+// the FP64 chains at 15 warps per SM, the registers' limit: 54-55 % of issue slots
+// and 49-50 % of the FP64 pipe; of 7 warp cycles per instruction 1.6 wait on a
+// fixed latency, 1.0 at a barrier, 0.6 for the FP64 pipe, 0.6 for global
 // loads.  So the gains lie in fewer instructions and no spills.  Measured per
 // 256^3 step on one box: 4.68 ms with a code path per axis, every bound by fmax
 // and fluxes over the primitives (a fourth barrier); 4.64 with both axes in one
