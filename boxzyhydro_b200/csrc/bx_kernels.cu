@@ -101,10 +101,13 @@ __device__ __forceinline__ void get_gamma2(const EosDev& e, double& eps, double 
 // Loads of the stage inputs: plain ones where the launch waits for the one before it
 // (grid_wait; not the read-only path, whose data may not change once a kernel has
 // started), from L2 (cg) in the persistent batched kernel, whose other blocks write
-// planes that this block reads later in the same launch.
-template <bool CG = false>
+// planes that this block reads later in the same launch.  __ldca and not *p: stage 1 of
+// the 256^3 box is 0.6 % slower with *p; but the force instances' stage 1 stores 76 and
+// 108 bytes of spills a thread with __ldca (power-of-two spacings and others), 44 and 68
+// with *p, and 8 steps of a 96^3 box with a potential take 3674 against 3644 us.
+template <bool CG = false, bool GRAV = false>
 __device__ __forceinline__ double ldg(const double* p) {
-  return CG ? __ldcg(p) : __ldca(p);
+  return CG ? __ldcg(p) : GRAV ? *p : __ldca(p);
 }
 
 // donor of a coordinate along one axis for a face ghost (fused path)
@@ -139,15 +142,15 @@ __device__ __forceinline__ Place place_of(const Geom& g, int x, int y, int z) {
   return p;
 }
 
-template <bool CG = false>
+template <bool CG = false, bool GRAV = false>
 __device__ __forceinline__ Cons load_cons(const double* B, long long PS, const Place& p) {
   const double* b = B + p.c;
   Cons r;
-  r.d = ldg<CG>(b);
-  r.m1 = ldg<CG>(b + PS);
-  r.m2 = ldg<CG>(b + 2 * PS);
-  r.m3 = ldg<CG>(b + 3 * PS);
-  r.E = ldg<CG>(b + 4 * PS);
+  r.d = ldg<CG, GRAV>(b);
+  r.m1 = ldg<CG, GRAV>(b + PS);
+  r.m2 = ldg<CG, GRAV>(b + 2 * PS);
+  r.m3 = ldg<CG, GRAV>(b + 3 * PS);
+  r.E = ldg<CG, GRAV>(b + 4 * PS);
   if (p.fx) r.m1 = -r.m1;
   if (p.fy) r.m2 = -r.m2;
   if (p.fz) r.m3 = -r.m3;
@@ -158,13 +161,13 @@ __device__ __forceinline__ Cons load_cons(const double* B, long long PS, const P
 // interior cells, or the gravitational acceleration (a ghost reads its donor's,
 // reflected components negated like the momenta: the source update is exact
 // under reflecting m and g together)
-template <bool CG = false>
+template <bool CG = false, bool GRAV = false>
 __device__ __forceinline__ void load_vec(const double* U, long long PS, const Place& p, double& u1,
                                          double& u2, double& u3) {
   const double* b = U + p.c;
-  u1 = ldg<CG>(b);
-  u2 = ldg<CG>(b + PS);
-  u3 = ldg<CG>(b + 2 * PS);
+  u1 = ldg<CG, GRAV>(b);
+  u2 = ldg<CG, GRAV>(b + PS);
+  u3 = ldg<CG, GRAV>(b + 2 * PS);
   if (p.fx) u1 = -u1;
   if (p.fy) u2 = -u2;
   if (p.fz) u3 = -u3;
@@ -263,11 +266,11 @@ __device__ __forceinline__ Raw load_raw(const StageArgs& a, const Place& p, int 
   const long long PS = a.ncells_total;
   Raw r;
   if (stage_is0<STAGE>(rs)) {
-    r.c = load_cons<CG>(a.X, PS, p);
-    if (GRAV) load_vec<CG>(a.G, PS, p, r.v1, r.v2, r.v3);
+    r.c = load_cons<CG, GRAV>(a.X, PS, p);
+    if (GRAV) load_vec<CG, GRAV>(a.G, PS, p, r.v1, r.v2, r.v3);
   } else {
-    r.c = load_cons<CG>(a.Y, PS, p);
-    load_vec<CG>(a.U, PS, p, r.v1, r.v2, r.v3);
+    r.c = load_cons<CG, GRAV>(a.Y, PS, p);
+    load_vec<CG, GRAV>(a.U, PS, p, r.v1, r.v2, r.v3);
   }
   return r;
 }
@@ -967,9 +970,9 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const Tile& t, co
       double go1 = 0.0, go2 = 0.0, go3 = 0.0;  // the own cell's acceleration
       if (plane) {
         const Place p{o, false, false, false};
-        c0 = load_cons<CG>(a.X, PS, p);
-        if (!is0) c1 = load_cons<CG>(a.Y, PS, p);
-        if (GRAV) load_vec<CG>(a.G, PS, p, go1, go2, go3);
+        c0 = load_cons<CG, GRAV>(a.X, PS, p);
+        if (!is0) c1 = load_cons<CG, GRAV>(a.Y, PS, p);
+        if (GRAV) load_vec<CG, GRAV>(a.G, PS, p, go1, go2, go3);
       }
       if (plane) {
         double ft[5];
