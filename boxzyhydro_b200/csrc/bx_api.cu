@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <exception>
@@ -892,10 +893,17 @@ static int host_io_setup(bx_handle* h) {
   // with 32, 21.1 with the 8 chunks of the stage launches), but no thinner than 2^17
   // cells (5 MB, 0.1 ms of copying) up to 8 planes, below which a slab's ten launches
   // and events cost more than its copies: per step with 2, 4, 8 and 16 planes 3.23,
-  // 2.83, 2.76 and 2.95 ms at 128^3, 1.26, 1.00, 0.88 and 0.92 at 64^3
+  // 2.83, 2.76 and 2.95 ms at 128^3, 1.26, 1.00, 0.88 and 0.92 at 64^3.  On flat grids
+  // the pipeline's fill and drain, about three slabs' copies (0.8 ns a cell each way),
+  // weigh more than the 20 us a slab costs: naz / zc slabs and the fill come cheapest at
+  // zc = sqrt(2^13 naz / sz).  Per step without this (in brackets: with 2 planes a
+  // slab and 256 threads a tile) and with it: 128x128x16 744 (713) and 605 us,
+  // 200x200x12 1205 (1000) and 999, 200x200x20 1462 (1377) and 1329, 160x160x40 1611
+  // (1671) and 1570.
   const int naz = g.az1 - g.az0;
   const int thin = (int)std::min<long long>(8, ((1ll << 17) + g.sz - 1) / g.sz);
-  const int zc = std::max({2, thin, (naz + 63) / 64});
+  const int flat = (int)std::lround(std::sqrt(8192.0 * naz / (double)g.sz));
+  const int zc = std::max({2, std::min(thin, flat), (naz + 63) / 64});
   const std::vector<Tile> tiles = make_tiles(g, 0, 1, zc);
   CK(cudaMalloc((void**)&h->d_io_tiles, tiles.size() * sizeof(Tile)));
   CK(cudaMemcpy(h->d_io_tiles, tiles.data(), tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice));

@@ -54,3 +54,16 @@ def test_two_dimensional_grid_of_two_slabs():
     assert slabs(ga, st) == 2
     ga.close()
     gb.close()
+
+
+@pytest.mark.parametrize("dims,count", [((132, 132, 20), 6), ((204, 100, 24), 7),
+                                        ((204, 204, 9), 3)])
+def test_flat_grids_have_thin_slabs(dims, count):
+    """Few planes: thinner slabs than 8 planes or 2^17 cells, whose pipeline would be
+    two or three slabs long."""
+    st = small_random_box(nx=dims[0], ny=dims[1], nz=dims[2], walls=(0, 1, 1, 0, 0, 0), seed=24)
+    ga, gb = run_pair(st, 2, pinned=True, in_place=True)
+    assert ga.status()[1] == 1
+    assert slabs(ga, st) == count
+    ga.close()
+    gb.close()
